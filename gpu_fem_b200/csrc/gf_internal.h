@@ -140,7 +140,30 @@ constexpr int kMaxEC = 15;
 // and a row's x entries come from a shared-memory ring of the latest `ring`
 // positions' results (ring > 2 maxdist, maxdist = the largest position
 // distance between a row and a row it multiplies).
-enum { TRI_LEVEL = 0, TRI_DATAFLOW = 1 };
+//
+// A triangle solved by the register-fed level sweep (kind TRI_RING) keeps its
+// rows in level order (position p = 0..n-1) too. The kRingWarps warps of a CTA
+// form `groups` groups; group g solves the levels g, g + groups, ... Every
+// warp has its own list of passes, tasks[lists[h kRingWarps + warp] ...]: up
+// to 16 blocks of one row a pass, {row (-1: none, -2: the warp helps another
+// one with a long row), blocks | flags | helpers << 5 | rows that the other
+// CTAs solve in this level << 16, first block, byte offset of the row's
+// result in the ring (helpers: the warp they help)}. A list ends with
+// kRingPad empty passes. The values of a row's blocks follow each other in
+// `stream` (36 values a block; U rows start with U_ii^{-1}), 16 blocks at a
+// time in the order in which the lanes of a warp load them (ring_value_pos),
+// and slots[b] is the ring byte offset of the x entries that block b
+// multiplies. Ring slot 0 holds zeros.
+enum { TRI_LEVEL = 0, TRI_DATAFLOW = 1, TRI_RING = 2 };
+constexpr int kRingWarps = 24;
+constexpr int kRingCta = 4;  // CTAs of a cluster at most
+constexpr int kRingPad = 4;
+enum {
+  kRingFirst = 1 << 10,   // first pass of a row
+  kRingLast = 1 << 11,    // last pass of a row
+  kRingBegin = 1 << 12,   // first pass of a level: wait for the level before
+  kRingEnd = 1 << 13      // last pass of a level: report it
+};
 struct TriDesc {
   int nch;                       // chunks
   int stage;                     // bytes of the largest chunk (staging buffer size)
@@ -149,9 +172,14 @@ struct TriDesc {
                                  // chunks; dataflow: [nch+1]
   const unsigned char* stream;
   long long abytes;              // algorithmic bytes of one sweep (for timing)
-  int nsplit;                    // level: CTAs that share each chunk's rows (1 or 2)
+  int nsplit;                    // level, ring: CTAs that share each level's rows
   int kind;                      // TRI_LEVEL or TRI_DATAFLOW
-  int ring, maxdist;             // dataflow: ring slots (a power of two), dependency reach
+  int ring, maxdist;             // dataflow: ring slots (a power of two), dependency reach;
+                                 // ring sweep: ring slots
+  const int4* tasks;             // ring sweep
+  const int32_t* slots;
+  const int32_t* lists;
+  int nlev, nblocks, groups;     // ring sweep: levels, stored blocks, groups of warps
 };
 
 // Per-problem descriptor used by the batched solver kernels: block rows,

@@ -141,20 +141,23 @@ __device__ __forceinline__ void mbar_arrive_remote(unsigned addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr)
                : "memory");
 }
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // bounded wait with acquire at cluster scope; false if limit_ns passed first
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, unsigned parity,
                                                   unsigned long long limit_ns) {
   unsigned long long t0 = 0;
   unsigned n = 0;
   while (true) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
+    if (mbar_try_wait_cluster(bar, parity)) return true;
     if (n == 0) t0 = gtimer();  // read only once the first test fails (reading it is slow)
     if ((++n & 255u) == 0u && gtimer() - t0 > limit_ns) return false;
   }
@@ -873,25 +876,332 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
   if (split) cluster_barrier();
 }
 
-// One sweep of a batch: a cluster of kSweepCta CTAs per problem.
+// --------------------------------------------- register-fed level sweeps
+// The default sweep. What bounds a level is the latency of its chain (x
+// entries -> products -> reduction -> U_ii^{-1} -> result -> barrier), so the
+// chain holds nothing else:
+//  - every x entry a triangle still needs sits in a shared-memory ring of
+//    the latest results (48 bytes a row; the ring covers the triangle's
+//    dependency reach), read straight into the products;
+//  - the warps form groups that take the levels in turn: while one group
+//    runs the chain of its level, the others load and convert the values of
+//    theirs. A level waits only for the level before it (bar.sync of its
+//    group against bar.arrive of the one before);
+//  - a warp takes a row 16 blocks a pass; lane (j, h) multiplies rows
+//    3h..3h+2 of block j. The values are read once, so they go from L2
+//    straight to registers while the other groups' levels run, and every pass
+//    prefetches as many bytes kRingAhead ahead of its own from HBM into L2;
+//  - the 16 partial sums of a row meet in a reduce-scatter of five 64-bit
+//    shuffles (a butterfly over three sums takes twelve);
+//  - rows of more than 16 blocks are shared by several warps.
+// In a triangle split over the CTAs of a cluster every result also goes to
+// the others' rings with st.async, whose bytes their mbarriers count per
+// level (bounded waits; no release of other stores is waited for).
+// Microseconds a level, chunked sweep -> this one (B200): 17x16 plate, ILU(8),
+// FP32 1.19 -> 0.56; 256x128, ILU(6), FP32 2.22 -> 0.85, FP64 3.54 -> 0.89;
+// 250x220, ILU(12), FP32 2.15 -> 0.92; 40x20, complete factor, FP64
+// 1.50 -> 0.58. Still latency-bound: ~120 dependent instructions a level.
+constexpr int kRingThreads = 32 * kRingWarps;
+constexpr size_t kRingSmemMax = 218 * 1024;  // dynamic; the static part is < 1 KB
+// Cost model of a level (clocks; it only chooses the layout), from applies of
+// 17x16 to 250x220 plates, ILU(6) to ILU(12) and complete factors: a chain
+// takes 0.56 us on one CTA and 0.73 us on two or four, a further round of
+// passes 0.85 us (its values are not there yet), each pass of a CTA some
+// issue slots; loading and converting hide behind the other groups' levels.
+constexpr double kRingChain = 1000.0, kRingSplit = 350.0, kRingRound = 1700.0, kRingIssue = 70.0,
+                 kRingPrep = 1300.0;
+constexpr int kRingAhead = 96 * 1024;  // bytes of values prefetched into L2 ahead of their use
+// rows up to which the chunked level sweep (bsweep_tma) always has a stage:
+// its chunk bound is then the base size of either precision
+constexpr int kRingRowAlways = 136;
+
+// position (in values, from the first value of the row's group of nb <= 16
+// blocks) of entry e = 6 r + c of block jj of the group; nb = 0: U_ii^{-1},
+// stored row-major. Lane 2 jj + r / 3 loads its 18 values as 16-byte pieces
+// (and one of 8 bytes in FP32), piece k of all lanes together.
+template <class VT>
+__host__ __device__ __forceinline__ int ring_value_pos(int nb, int jj, int e) {
+  if (nb == 0) return e;
+  constexpr int pv = 16 / (int)sizeof(VT);  // values of a 16-byte piece
+  constexpr int full = 18 / pv;             // whole pieces of a lane
+  const int r = e / 6, lane = 2 * jj + r / 3, v = 6 * (r % 3) + e % 6;
+  if (v < full * pv) return (v / pv * 2 * nb + lane) * pv + v % pv;
+  return full * 2 * nb * pv + lane * (18 - full * pv) + (v - full * pv);
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
+}
+// 8 bytes into another CTA's shared memory, counted on its mbarrier
+__device__ __forceinline__ void st_async(unsigned addr, double v, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                   addr),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void named_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void ring_load(const float* p, int lane, int n2, float (&v)[18]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(p) + k * n2 + lane);
+    v[4 * k] = q.x, v[4 * k + 1] = q.y, v[4 * k + 2] = q.z, v[4 * k + 3] = q.w;
+  }
+  const float2 q = __ldg(reinterpret_cast<const float2*>(p + 16 * n2) + lane);
+  v[16] = q.x, v[17] = q.y;
+}
+__device__ __forceinline__ void ring_load(const double* p, int lane, int n2, double (&v)[18]) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const double2 q = __ldg(reinterpret_cast<const double2*>(p) + k * n2 + lane);
+    v[2 * k] = q.x, v[2 * k + 1] = q.y;
+  }
+}
+// volatile: the conversions stay ahead of the barrier that follows them
+__device__ __forceinline__ void ring_take(const float (&v)[18], double (&d)[18]) {
+#pragma unroll
+  for (int k = 0; k < 18; k++) asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d[k]) : "f"(v[k]));
+}
+__device__ __forceinline__ void ring_take(const double (&v)[18], double (&d)[18]) {
+#pragma unroll
+  for (int k = 0; k < 18; k++) d[k] = v[k];
+}
+
 template <class VT, bool UPPER>
-static cudaError_t launch_sweep(int np, size_t smem, cudaStream_t st, const ProbDev* desc,
-                                const int* live, const double* rhs, double* out, SweepCtl* ctl,
+__global__ void __launch_bounds__(kRingThreads, 1)
+    bsweep_ring(const ProbDev* __restrict__ P, const int* __restrict__ live,
+                const double* __restrict__ rhs, double* out, SweepCtl* ctl,
+                unsigned long long* bytes_ctr) {
+  extern __shared__ __align__(128) unsigned char ring[];
+  __shared__ uint64_t xbar[2];  // the other CTAs' results of even / odd levels
+  __shared__ double part[kRingWarps][6];  // a helper's sums for the row's warp
+  __shared__ volatile int abort_flag;
+  unsigned ncta;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+  const int p = blockIdx.x / ncta;
+  const unsigned rank = cluster_rank();
+  if (live && !live[p]) return;  // the same for every CTA of the cluster
+  const TriDesc& T = UPPER ? P[p].U : P[p].L;
+  if (T.kind != TRI_RING) return;
+  const int nsplit = T.nsplit;
+  // CTAs without rows leave at once (a cluster barrier counts only threads
+  // that have not exited, and no other CTA writes here)
+  if ((int)rank >= nsplit) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = lane & 1;
+  const bool split = nsplit > 1;
+  if (tid == 0) {
+    mbar_init(&xbar[0], 1);
+    mbar_init(&xbar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    abort_flag = 0;
+  }
+  if (tid < 6) reinterpret_cast<double*>(ring)[tid] = 0.0;
+  if (split)
+    cluster_barrier();  // every CTA's barriers exist before any remote store
+  else
+    __syncthreads();
+  const bool send = split && !(g_skip_meet && rank == 1);
+  const double* rb = rhs + 6 * (size_t)P[p].off;
+  double* ob = out + 6 * (size_t)P[p].off;
+  const unsigned char* stream = T.stream;
+  const VT* vals = reinterpret_cast<const VT*>(stream);
+  const int32_t* slots = T.slots;
+  const int groups = T.groups, wpg = kRingWarps / groups, nlev = T.nlev;
+  const int gi = warp / wpg;  // the warp's group
+  const bool lead = warp == gi * wpg && lane == 0;
+  // barriers of the level before (of this group) and of this group's
+  // levels; the others serve rows that several warps share
+  const int bar_in = 1 + (gi ? gi - 1 : groups - 1), bar_out = 1 + gi;
+  const int bar_threads = 64 * wpg;
+  const size_t vbytes = (size_t)T.nblocks * 36 * sizeof(VT);
+  for (size_t a = 128 * (size_t)tid; a < min(vbytes, (size_t)kRingAhead); a += 128 * kRingThreads)
+    prefetch_l2(stream + a);
+  // the row (of the block's six) whose sum ends in this lane, and whether
+  // the lane writes it
+  const int rr = 3 * h + ((lane & 16) ? 2 : (lane & 8) ? 1 : 0);
+  const bool writer = (lane & 6) == 0 && (lane & 24) != 24;
+  const bool b4 = lane & 16, b3 = lane & 8;
+  const int4* tasks = T.tasks + T.lists[rank * kRingWarps + warp];
+  VT v[18];  // values of this pass
+  VT di[6];  // row rr of U_ii^{-1}
+  double acc[3] = {0.0, 0.0, 0.0}, rv = 0.0;
+  int slot = 0;  // ring offset of this lane's x entries
+#pragma unroll
+  for (int k = 0; k < 6; k++) di[k] = (VT)0;
+  auto load = [&](const int4& t) {
+    const int nb = t.y & 31;
+    slot = 0;
+#pragma unroll
+    for (int k = 0; k < 18; k++) v[k] = (VT)0;
+    if (lane < 2 * nb) {
+      slot = __ldg(slots + t.z + (lane >> 1));
+      ring_load(vals + 36 * (size_t)t.z, lane, 2 * nb, v);
+      const size_t a = 36 * sizeof(VT) * (size_t)t.z + kRingAhead + 128 * (size_t)lane;
+      if (lane * 128 < 36 * (int)sizeof(VT) * nb + 127 && a < vbytes) prefetch_l2(stream + a);
+    }
+    if (t.x >= 0 && (t.y & kRingFirst)) {
+      rv = rb[6 * (size_t)t.x + rr];
+      if (UPPER) {
+        using V2 = typename std::conditional<sizeof(VT) == 8, double2, float2>::type;
+        // U_ii^{-1} precedes the row's first block
+        const V2* q = reinterpret_cast<const V2*>(vals + 36 * (size_t)(t.z - 1) + 6 * rr);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const V2 u = __ldg(q + k);
+          di[2 * k] = u.x, di[2 * k + 1] = u.y;
+        }
+      }
+    }
+  };
+  int4 t0 = __ldg(tasks), t1 = __ldg(tasks + 1);
+  tasks += 2;
+  load(t0);
+  int lev = gi;  // this group's level
+  while (lev < nlev) {
+    const int4 t2 = __ldg(tasks++);
+    double d[18];
+    ring_take(v, d);
+    if (t0.y & kRingFirst) acc[0] = acc[1] = acc[2] = 0.0;
+    if (t0.y & kRingBegin) {
+      if (lev > 0) {
+        named_sync(bar_in, bar_threads);
+        if (split && !abort_flag) {
+          uint64_t* b = &xbar[(lev - 1) & 1];
+          const unsigned par = (unsigned)(((lev - 1) >> 1) & 1);
+          unsigned long long w0 = 0;
+          while (!mbar_try_wait_cluster(b, par)) {
+            if (abort_flag) break;
+            if (w0 == 0) w0 = gtimer();
+            if (gtimer() - w0 > g_wait_ns) abort_flag = 1;
+          }
+        }
+      }
+      if (split && lead && !abort_flag)
+        mbar_expect_tx(&xbar[lev & 1], 48u * ((unsigned)t0.y >> 16));
+    }
+    if (t0.x != -1) {
+      {
+        // lanes without a block multiply zeros
+        const double2* x = reinterpret_cast<const double2*>(ring + slot);
+        const double2 x0 = x[0], x1 = x[1], x2 = x[2];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          acc[r] = fma(d[6 * r], x0.x, acc[r]);
+          acc[r] = fma(d[6 * r + 1], x0.y, acc[r]);
+          acc[r] = fma(d[6 * r + 2], x1.x, acc[r]);
+          acc[r] = fma(d[6 * r + 3], x1.y, acc[r]);
+          acc[r] = fma(d[6 * r + 4], x2.x, acc[r]);
+          acc[r] = fma(d[6 * r + 5], x2.y, acc[r]);
+        }
+      }
+      if (t0.y & kRingLast) {
+        // lanes with bit 4 keep row 2, the others rows 0 and 1; those split
+        // on bit 3
+        const double y0 = __shfl_xor_sync(0xffffffffu, b4 ? acc[0] : acc[2], 16);
+        const double y1 = __shfl_xor_sync(0xffffffffu, acc[1], 16);
+        const double k0 = (b4 ? acc[2] : acc[0]) + y0, k1 = acc[1] + y1;
+        const double y2 = __shfl_xor_sync(0xffffffffu, b4 || b3 ? k0 : k1, 8);
+        double a = (b4 || !b3 ? k0 : k1) + y2;
+        a += __shfl_xor_sync(0xffffffffu, a, 4);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        const int helpers = (t0.y >> 5) & 31;
+        if (t0.x == -2) {  // this warp helps warp t0.w with its row
+          if (writer) part[warp][rr] = a;
+          named_arrive((1 + groups + t0.w / 2) & 15, 32 * (helpers + 1));
+        } else {
+          if (helpers) {
+            named_sync((1 + groups + warp / 2) & 15, 32 * (helpers + 1));
+            for (int k = 1; k <= helpers; k++) a += part[warp + k][rr];
+          }
+          double z = rv - a;
+          if (UPPER) {
+            double tc[6];
+#pragma unroll
+            for (int c = 0; c < 6; c++)
+              tc[c] = __shfl_sync(0xffffffffu, z, c / 3 + (c % 3 == 2 ? 16 : 8 * (c % 3)));
+            z = fma((double)di[4], tc[4], fma((double)di[2], tc[2], (double)di[0] * tc[0])) +
+                fma((double)di[5], tc[5], fma((double)di[3], tc[3], (double)di[1] * tc[1]));
+          }
+          if (writer) {
+            const unsigned o = (unsigned)t0.w + 8u * (unsigned)rr;
+            *reinterpret_cast<double*>(ring + o) = z;
+            if (send)
+              for (int q = 1; q < nsplit; q++) {
+                const unsigned c = (rank + q) & (nsplit - 1);
+                st_async(cluster_map(smem_u32(ring + o), c), z,
+                         cluster_map(smem_u32(&xbar[lev & 1]), c));
+              }
+            ob[6 * (size_t)t0.x + rr] = z;
+          }
+        }
+      }
+    }
+    if (t0.y & kRingEnd) {
+      if (lev + 1 < nlev) named_arrive(bar_out, bar_threads);
+      lev += groups;
+    }
+    t0 = t1;
+    t1 = t2;
+    load(t0);
+  }
+  if (split) {
+    // the other CTAs' results of the last level have landed (nothing may
+    // be in flight into a CTA that ends)
+    __syncthreads();
+    if (tid == 0 && !abort_flag &&
+        !mbar_wait_cluster(&xbar[(nlev - 1) & 1], (unsigned)(((nlev - 1) >> 1) & 1), g_wait_ns))
+      abort_flag = 1;
+    if (tid == 0 && abort_flag) atomicOr(&ctl->status, ST_TIMEOUT);
+  }
+  if (tid == 0 && rank == 0 && bytes_ctr && !abort_flag)
+    atomicAdd(bytes_ctr, (unsigned long long)T.abytes);
+  if (split) {
+    // no CTA leaves while another may still write into its ring; every path
+    // of every CTA of a split problem reaches this point
+    __syncthreads();
+    cluster_barrier();
+  }
+}
+
+// Factor values into a ring sweep's stream: block q of the triangle takes
+// the 6x6 block src[map[q]]; code[q] = (blocks of its group << 8) + its
+// number in the group (0 for U_ii^{-1}).
+template <class VT>
+__global__ void repack_ring_kernel(size_t nblocks, const int32_t* __restrict__ map,
+                                   const uint16_t* __restrict__ code,
+                                   const double* __restrict__ src, VT* __restrict__ dst) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nblocks * 36) return;
+  const size_t q = t / 36;
+  const int e = (int)(t % 36), nb = code[q] >> 8, jj = code[q] & 255;
+  dst[36 * (q - jj) + ring_value_pos<VT>(nb, jj, e)] = (VT)src[36 * (size_t)map[q] + e];
+}
+
+// One sweep of a batch: a cluster of `ctas` CTAs per problem.
+typedef void (*SweepKernel)(const ProbDev*, const int*, const double*, double*, SweepCtl*,
+                            unsigned long long*);
+static cudaError_t launch_sweep(SweepKernel kernel, int ctas, int threads, int np, size_t smem,
+                                cudaStream_t st, const ProbDev* desc, const int* live,
+                                const double* rhs, double* out, SweepCtl* ctl,
                                 unsigned long long* ctr) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(np * kSweepCta));
-  cfg.blockDim = dim3(kSweepThreads);
+  cfg.gridDim = dim3((unsigned)(np * ctas));
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kSweepCta;
+  attr[0].val.clusterDim.x = (unsigned)ctas;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   ::gf::count_launch();
-  return cudaLaunchKernelEx(&cfg, bsweep_tma<VT, UPPER>, desc, live, rhs, out, ctl, ctr);
+  return cudaLaunchKernelEx(&cfg, kernel, desc, live, rhs, out, ctl, ctr);
 }
 
 // ------------------------------------------------------ dataflow sweeps
@@ -1492,6 +1802,10 @@ struct gf_precond {
     DevBuf<int64_t> off, vpos;
     DevBuf<int32_t> map;
     DevBuf<unsigned char> stream;
+    int nlev = 0, groups = 0;     // ring sweep
+    DevBuf<int4> tasks;
+    DevBuf<int32_t> slots, lists;
+    DevBuf<uint16_t> code;
   } tri[2];  // 0 = L, 1 = U
   gf_batch* self = nullptr;  // batch of one, built on first use
 };
@@ -1854,13 +2168,176 @@ static cudaError_t build_df(gf_precond* p, const std::vector<int32_t>& diag, boo
   if (e == cudaSuccess) *used = true;
   return e;
 }
+// Streams of one triangle for the register-fed level sweep (layout described
+// at TriDesc). Returns cudaSuccess with *used = false, building nothing, when
+// the ring would not fit one CTA's shared memory.
+static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, bool upper,
+                              bool* used) {
+  const Pattern& P = p->pat;
+  const int n = P.n;
+  const std::vector<int32_t>& lv = upper ? p->lvU : p->lvL;
+  const int nlev = upper ? p->nlevU : p->nlevL;
+  const size_t vs = p->prec == GF_PREC_FP32 ? 4 : 8;
+  const int first = upper ? 1 : 0;
+  *used = false;
+  auto beg = [&](int i) { return upper ? diag[i] + 1 : P.rowp[i]; };
+  auto end = [&](int i) { return upper ? P.rowp[i + 1] : diag[i]; };
+  std::vector<int32_t> ptr(nlev + 1, 0), rows(n), pos(n);
+  for (int i = 0; i < n; i++) ptr[lv[i] + 1]++;
+  int maxlev = 0;
+  for (int l = 0; l < nlev; l++) {
+    maxlev = std::max(maxlev, ptr[l + 1]);
+    ptr[l + 1] += ptr[l];
+  }
+  {
+    std::vector<int32_t> f(ptr.begin(), ptr.end() - 1);
+    for (int i = 0; i < n; i++) {
+      pos[i] = f[lv[i]]++;
+      rows[pos[i]] = i;
+    }
+  }
+  int maxdist = 0;
+  for (int i = 0; i < n; i++)
+    for (int jp = beg(i); jp < end(i); jp++) maxdist = std::max(maxdist, pos[i] - pos[P.cols[jp]]);
+  // while rows of level l are still being solved the partner may already
+  // write rows of level l + 1
+  const long long ring = (long long)maxdist + 2ll * maxlev + 1;
+  if ((ring + 1) * 48 > (long long)kRingSmemMax || maxlev > 0xffff) return cudaSuccess;
+  auto slot = [&](int i) { return (int)(pos[i] % ring + 1) * 48; };  // slot 0 holds zeros
+  // CTAs and groups of warps (clocks on B200): a level costs its chain, a
+  // further round for passes beyond one per warp, and the issue slots of its
+  // passes; a split adds the exchange
+  auto model = [&](int ns, int groups) {
+    const int wpg = kRingWarps / groups;
+    double cyc = 0.0;
+    for (int l = 0; l < nlev; l++) {
+      int passes = 0;
+      for (int k = ptr[l]; k < ptr[l + 1]; k++)
+        passes += std::max(1, (end(rows[k]) - beg(rows[k]) + 15) / 16);
+      const int per = (passes + ns - 1) / ns, rounds = (per + wpg - 1) / wpg;
+      const double chain = kRingChain + (upper ? 90.0 : 0.0) + (ns > 1 ? kRingSplit : 0.0) +
+                           kRingRound * (rounds - 1.0) + kRingIssue * per;
+      cyc += std::max(chain, (chain + kRingPrep) / groups);
+    }
+    return cyc;
+  };
+  int nsplit = 1, groups = 2;
+  double best = 1e300;
+  for (int ns = 1; ns <= kRingCta; ns *= 2)
+    for (int g = 2; g <= 3; g++)
+      if (model(ns, g) < best) {
+        best = model(ns, g);
+        nsplit = ns;
+        groups = g;
+      }
+  const int wpg = kRingWarps / groups;
+  size_t nblocks = (size_t)first * n;
+  for (int i = 0; i < n; i++) nblocks += end(i) - beg(i);
+  std::vector<int32_t> slots(nblocks + 4, 0), map(nblocks);
+  std::vector<uint16_t> code(nblocks);
+  std::vector<std::vector<int4>> lists((size_t)kRingCta * kRingWarps);
+  size_t b = 0;
+  std::vector<int32_t> mine[kRingCta];
+  long long npass = 0;
+  for (int l = 0; l < nlev; l++) {
+    // a level's rows over the CTAs: each to the one with fewer blocks so far
+    // (ties: fewer rows)
+    long long hb[kRingCta] = {0};
+    for (auto& m : mine) m.clear();
+    for (int k = ptr[l]; k < ptr[l + 1]; k++) {
+      int h = 0;
+      for (int q = 1; q < nsplit; q++)
+        if (hb[q] < hb[h] || (hb[q] == hb[h] && mine[q].size() < mine[h].size())) h = q;
+      hb[h] += end(rows[k]) - beg(rows[k]) + first;
+      mine[h].push_back(rows[k]);
+    }
+    for (int h = 0; h < nsplit; h++) {
+      const int others = ptr[l + 1] - ptr[l] - (int)mine[h].size();
+      const int w0 = h * kRingWarps + (l % groups) * wpg;
+      // lists of the group's warps, this level's part
+      size_t start[kRingWarps];
+      for (int w = 0; w < wpg; w++) start[w] = lists[w0 + w].size();
+      // rows of several passes are shared while every row still finds warps
+      // of its own (a barrier of helpers is used once a level); the others
+      // take their passes one after another
+      int w = 0, left = (int)mine[h].size();
+      for (int i : mine[h]) {
+        const int nb = end(i) - beg(i), np = std::max(1, (nb + 15) / 16);
+        left--;
+        const int room = wpg - w - left;  // 0 or less once a second round began
+        const int segs = std::max(1, std::min(np, room));
+        int pass = 0;
+        for (int q = 0; q < segs; q++) {
+          auto& L = lists[w0 + w % wpg + q];
+          const int p1 = np * (q + 1) / segs;
+          if (upper && q == 0) {
+            map[b] = diag[i];
+            code[b++] = 0;
+          }
+          for (int p0 = pass; pass < p1; pass++) {
+            const int j0 = 16 * pass, m = std::min(16, nb - j0);
+            const int flags = (pass == p0 ? kRingFirst : 0) |
+                              (pass + 1 == p1 ? kRingLast | (segs - 1) << 5 : 0);
+            L.push_back(make_int4(q ? -2 : i, m | flags, (int)b,
+                                  q ? (l % groups) * wpg + w : slot(i)));
+            for (int j = 0; j < m; j++) {
+              const int jp = beg(i) + j0 + j;
+              map[b] = jp;
+              slots[b] = slot(P.cols[jp]);
+              code[b++] = (uint16_t)(m << 8 | j);
+            }
+          }
+        }
+        w += segs;
+      }
+      for (int q = 0; q < wpg; q++) {
+        auto& L = lists[w0 + q];
+        if (L.size() == start[q]) L.push_back(make_int4(-1, 0, (int)b, 0));
+        L[start[q]].y |= kRingBegin | others << 16;
+        L.back().y |= kRingEnd;
+        npass = std::max(npass, (long long)L.size());
+      }
+    }
+  }
+  std::vector<int4> all;
+  std::vector<int32_t> where;
+  for (auto& L : lists) {
+    where.push_back((int32_t)all.size());
+    all.insert(all.end(), L.begin(), L.end());
+    all.insert(all.end(), kRingPad, make_int4(-1, 0, 0, 0));
+  }
+  gf_precond::Tri& t = p->tri[upper ? 1 : 0];
+  t.kind = TRI_RING;
+  t.nsplit = nsplit;
+  t.groups = groups;
+  t.ring = (int)ring;
+  t.maxdist = maxdist;
+  t.nch = (int)npass;
+  t.nlev = nlev;
+  t.nslots = nblocks;
+  t.abytes = (long long)nblocks * (36 * (long long)vs + 4) + (long long)n * (4 + 48 + 48) + 4;
+  cudaError_t e = cudaSuccess;
+  auto up = [&](cudaError_t x) {
+    if (e == cudaSuccess) e = x;
+  };
+  up(t.tasks.upload(all));
+  up(t.slots.upload(slots));
+  up(t.lists.upload(where));
+  up(t.map.upload(map));
+  up(t.code.upload(code));
+  up(t.stream.alloc(nblocks * 36 * vs));
+  if (e == cudaSuccess) *used = true;
+  return e;
+}
 static TriDesc tri_desc(const gf_precond* p, int which) {
   const gf_precond::Tri& t = p->tri[which];
-  return TriDesc{t.nch,    t.stage,  t.capb, t.capr, t.off.p,   t.stream.p,
-                 t.abytes, t.nsplit, t.kind, t.ring, t.maxdist};
+  return TriDesc{t.nch,    t.stage,  t.capb,    t.capr,    t.off.p,   t.stream.p, t.abytes,
+                 t.nsplit, t.kind,   t.ring,    t.maxdist, t.tasks.p, t.slots.p,  t.lists.p,
+                 t.nlev,   (int)t.nslots, t.groups};
 }
 static size_t sweep_smem(const gf_precond* p, int which) {
   const gf_precond::Tri& t = p->tri[which];
+  if (t.kind == TRI_RING) return 48 * ((size_t)t.ring + 1);
   return t.kind == TRI_DATAFLOW ? df_smem_bytes(t.stage, t.ring)
                                 : sweep_smem_bytes(t.stage, t.capb, t.capr);
 }
@@ -1869,8 +2346,11 @@ static size_t sweep_smem(const gf_precond* p, int which) {
 struct gf_batch {
   int np = 0, nrows = 0, maxlevL = 0, maxlevU = 0;
   size_t smemL = 0, smemU = 0;  // dynamic shared memory of the level-synchronous sweeps
-  size_t dfL = 0, dfU = 0;      // ... and of the dataflow sweeps
-  int nlevelL = 0, nlevelU = 0, ndfL = 0, ndfU = 0;  // problems solved by each kind
+  size_t dfL = 0, dfU = 0;      // ... of the dataflow sweeps
+  size_t ringL = 0, ringU = 0;  // ... and of the register-fed level sweeps
+  // problems solved by each kind
+  int nlevelL = 0, nlevelU = 0, ndfL = 0, ndfU = 0, nringL = 0, nringU = 0;
+  int ctasL = 1, ctasU = 1;      // cluster size of the register-fed sweeps
   int pprec = GF_PREC_FP64;      // factor precision shared by the batch's preconditioners
   size_t N = 0;  // doubles in batch space
   std::vector<gf_assembler*> asms;
@@ -2106,10 +2586,18 @@ static gf_status batch_build(gf_batch* B) {
   for (int k = 0; k < np; k++) {
     if (B->pcs[k]->prec != B->pprec) return GF_INVALID_ARG;  // one factor precision per batch
     for (int w = 0; w < 2; w++) {
-      const bool df = B->pcs[k]->tri[w].kind == TRI_DATAFLOW;
-      size_t& sm = df ? (w ? B->dfU : B->dfL) : (w ? B->smemU : B->smemL);
+      const int kind = B->pcs[k]->tri[w].kind;
+      size_t& sm = kind == TRI_DATAFLOW ? (w ? B->dfU : B->dfL)
+                   : kind == TRI_RING   ? (w ? B->ringU : B->ringL)
+                                        : (w ? B->smemU : B->smemL);
       sm = std::max(sm, sweep_smem(B->pcs[k], w));
-      (df ? (w ? B->ndfU : B->ndfL) : (w ? B->nlevelU : B->nlevelL))++;
+      if (kind == TRI_RING) {
+        int& c = w ? B->ctasU : B->ctasL;
+        c = std::max(c, B->pcs[k]->tri[w].nsplit);
+      }
+      (kind == TRI_DATAFLOW ? (w ? B->ndfU : B->ndfL)
+       : kind == TRI_RING   ? (w ? B->nringU : B->nringL)
+                            : (w ? B->nlevelU : B->nlevelL))++;
     }
     for (int i = 0; i < B->asms[k]->nnodes; i++) row_prob[B->offs[k] + i] = k;
     B->maxlevL = std::max(B->maxlevL, B->pcs[k]->nlevL);
@@ -2286,8 +2774,16 @@ static cudaError_t launch_tri(gf_batch* B, cudaStream_t st, const int* live, con
     e = cudaFuncSetAttribute(bsweep_tma<VT, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSweepSmemMax);
     if (e != cudaSuccess) return e;
-    e = launch_sweep<VT, UPPER>(B->np, UPPER ? B->smemU : B->smemL, st, B->d_desc.p, live, rhs,
-                                out, B->d_ctl.p, ctr);
+    e = launch_sweep(bsweep_tma<VT, UPPER>, kSweepCta, kSweepThreads, B->np, UPPER ? B->smemU : B->smemL, st,
+                     B->d_desc.p, live, rhs, out, B->d_ctl.p, ctr);
+    if (e != cudaSuccess) return e;
+  }
+  if (UPPER ? B->nringU : B->nringL) {
+    e = cudaFuncSetAttribute(bsweep_ring<VT, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSweepSmemMax);
+    if (e != cudaSuccess) return e;
+    e = launch_sweep(bsweep_ring<VT, UPPER>, UPPER ? B->ctasU : B->ctasL, kRingThreads, B->np,
+                     UPPER ? B->ringU : B->ringL, st, B->d_desc.p, live, rhs, out, B->d_ctl.p, ctr);
   }
   return e;
 }
@@ -2384,6 +2880,16 @@ static gf_status batch_factor(gf_batch* B, cudaStream_t st) {
       gf_precond::Tri& t = p->tri[w];
       const unsigned nb = (unsigned)((t.nslots * 36 + 255) / 256);
       if (t.nslots == 0) continue;
+      if (t.kind == TRI_RING) {
+        if (p->prec == GF_PREC_FP32)
+          repack_ring_kernel<float><<<nb, 256, 0, st>>>(t.nslots, t.map.p, t.code.p, p->d_lu.p,
+                                                        reinterpret_cast<float*>(t.stream.p));
+        else
+          repack_ring_kernel<double><<<nb, 256, 0, st>>>(t.nslots, t.map.p, t.code.p, p->d_lu.p,
+                                                         reinterpret_cast<double*>(t.stream.p));
+        ::gf::count_launch();
+        continue;
+      }
       if (p->prec == GF_PREC_FP32)
         repack_kernel<float><<<nb, 256, 0, st>>>(t.nslots, t.map.p, t.vpos.p, p->d_lu.p,
                                                   reinterpret_cast<float*>(t.stream.p));
@@ -2776,6 +3282,26 @@ gf_status gf_precond_create_ex(gf_assembler* a, int32_t fill_level, int32_t prec
   for (int w = 0; w < 2 && e == cudaSuccess; w++) {
     bool df = false;
     if (sweep == GF_SWEEP_DATAFLOW) e = build_df(p, diag, w == 1, &df);
+    // the factors that are refused for their longest row are those that the
+    // chunked level sweep cannot stage, whichever sweep solves them: short
+    // rows always fit, others are laid out to see
+    if (sweep == GF_SWEEP_AUTO) {
+      int most = 0;
+      for (int i = 0; i < n; i++)
+        most = std::max(most, w ? p->pat.rowp[i + 1] - diag[i] : diag[i] - p->pat.rowp[i]);
+      if (most > kRingRowAlways) {
+        e = build_tri(p, diag, w == 1);
+        if (e == cudaSuccess && sweep_smem(p, w) > kSweepSmemMax) break;
+      }
+      if (e == cudaSuccess) e = build_ring(p, diag, w == 1, &df);
+      if (df) {  // the chunked stream, where it was built
+        gf_precond::Tri& t = p->tri[w];
+        t.off.release();
+        t.vpos.release();
+      } else if (e == cudaSuccess && most > kRingRowAlways) {
+        continue;
+      }
+    }
     if (e == cudaSuccess && !df) {
       if (sweep == GF_SWEEP_DATAFLOW) {
         set_last_error_text("gf_precond_create_ex: the dataflow sweep's ring and stages of this "
@@ -2833,8 +3359,8 @@ gf_status gf_precond_setup_info(const gf_precond* p, int32_t* symbolic_on_gpu, d
 gf_status gf_precond_layout(const gf_precond* p, int32_t* nsplit_L, int32_t* nsplit_U,
                             int32_t* fac_ctas, int32_t* chunks_L, int32_t* chunks_U) {
   if (!p) return GF_INVALID_ARG;
-  if (nsplit_L) *nsplit_L = p->tri[0].nsplit;
-  if (nsplit_U) *nsplit_U = p->tri[1].nsplit;
+  if (nsplit_L) *nsplit_L = std::min(p->tri[0].nsplit, 2);
+  if (nsplit_U) *nsplit_U = std::min(p->tri[1].nsplit, 2);
   if (fac_ctas) *fac_ctas = fac_ctas_alone(p);
   if (chunks_L) *chunks_L = p->tri[0].nch;
   if (chunks_U) *chunks_U = p->tri[1].nch;
@@ -2849,8 +3375,9 @@ gf_status gf_precond_sweeps(const gf_precond* p, int32_t* kind_L, int32_t* kind_
   };
   if (kind_L) *kind_L = kind(p->tri[0]);
   if (kind_U) *kind_U = kind(p->tri[1]);
-  if (ring_L) *ring_L = p->tri[0].ring;
-  if (ring_U) *ring_U = p->tri[1].ring;
+  auto slots = [](const gf_precond::Tri& t) { return t.kind == TRI_DATAFLOW ? t.ring : 0; };
+  if (ring_L) *ring_L = slots(p->tri[0]);
+  if (ring_U) *ring_U = slots(p->tri[1]);
   return GF_OK;
 }
 

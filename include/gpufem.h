@@ -241,8 +241,12 @@ gf_status gf_precond_create(gf_assembler* a, int32_t fill_level, int32_t precisi
  *                     when a chunk-cost model says it pays (levels with
  *                     more rows than one CTA's warps or more blocks than its
  *                     stage);
- *  GF_SWEEP_AUTO      the level-synchronous kernel (the faster of the two
- *                     on the batched plate workload on B200).
+ *  GF_SWEEP_AUTO      a level-ordered kernel that keeps the results a
+ *                     triangle still reads in shared memory and the factor
+ *                     values in registers (2 to 4 times as fast as
+ *                     GF_SWEEP_LEVEL on B200); GF_SWEEP_LEVEL's kernel where
+ *                     the dependency reach does not fit (about 4600 rows).
+ *                     Reported as GF_SWEEP_LEVEL.
  * The dataflow kernel needs its result ring and stages to fit one CTA's
  * shared memory: a factor whose rows reach back more than ~1000 positions
  * in level order does not fit.
@@ -296,11 +300,13 @@ gf_status gf_precond_apply_noalloc(gf_precond* p, const double* d_r, double* d_z
  * errors, include/cuda_utils.h:35-43). */
 gf_status gf_precond_status(gf_precond* p, void* stream);
 /* How the triangular work of this preconditioner is laid out on the GPU:
- * CTAs that share each sweep chunk's rows (1 or 2) for L and U, the CTAs the
+ * whether one CTA solves a sweep's rows (1) or the CTAs of a cluster share
+ * those of every level (2) for L and U, the CTAs the
  * dataflow factorization runs on when this preconditioner is factored alone
  * (1 to 128; in a batch the SMs are shared out by the problems' block
  * updates), and the number of chunks of each triangle (a chunk holds rows of one level; a
- * level with more blocks than a chunk's stage spans several). Any pointer
+ * level with more blocks than a chunk's stage spans several; in the default
+ * sweep the passes of its busiest warp). Any pointer
  * may be NULL. No reference counterpart (cuSPARSE's bsrsv2 level analysis is
  * internal). */
 /* Where and how long the preconditioner's setup ran: whether its ILU(k)
