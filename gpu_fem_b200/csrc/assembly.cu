@@ -5,285 +5,668 @@
 // scatter with FP64 atomicAdd (include/linalg/vec.h:278-293,
 // include/linalg/bsr_mat.h:229-276).
 //
-// Here a warp owns a chunk of up to eight neighbouring elements:
-//   * coordinates and DOFs of the chunk are gathered into the warp's shared
-//     memory slot and the per-element geometry (normals, nodal frames, the
-//     four quadrature-point frames, the tying-point vectors) is computed by
-//     8 x 4 lanes at once;
-//   * per element, lane l < 24 builds column l of the four 9x24 strain
-//     matrices B_q and of D B_q; each of the 32 lanes then owns a 3x6 tile of
-//     K_e = sum_q B_q^T D B_q (144 contiguous bytes of one 6x6 BSR block) and
-//     writes it with 16-byte stores; R_e = K_e u_e follows from the tiles;
+// Here a CTA of four warps owns a chunk of up to eight neighbouring elements:
+//   * the chunk's coordinates and DOFs are gathered into shared memory; the
+//     node normals, the frames of the four nodes and of the four quadrature
+//     points are computed with one lane per (element, point);
+//   * a warp tabulates its element's 24 columns (ElemData); lane (i, q) then
+//     evaluates the strains of columns i, 8 + i, 16 + i at quadrature point q
+//     and K_e = sum_q B_q^T D B_q is accumulated by FP64 tensor instructions
+//     (mma.m8n8k4) whose contraction index is the quadrature point, one
+//     strain component a step: the operands are the lane's own values, so no
+//     strain matrix is ever stored. K_e is symmetric: six of nine 8x8 tiles,
+//     the others are mirrored as they go to shared memory;
+//   * the chunk's elements are summed block by block from shared memory, in
+//     element order, and every block goes to global memory once per chunk;
 //   * the scatter follows the coloured schedule built on the host: chunks of
-//     one colour share no node and run concurrently (one launch per colour);
-//     inside a chunk the warp handles its elements in order. The first
-//     toucher of a block stores, later touchers read-modify-write; there are
-//     no atomics and the result is bitwise reproducible;
+//     one colour share no node and run concurrently, one launch per colour.
+//     The launches overlap (programmatic dependent launch): a chunk computes
+//     its K_e while the colour before still scatters, and waits only before
+//     its own scatter. The first colour that touches a block stores, later
+//     ones read-modify-write; there are no atomics and the result is bitwise
+//     reproducible;
 //   * with GF_ASSEMBLE_ATOMIC the colours are ignored: the outputs are zeroed
 //     and one launch over all chunks adds with FP64 atomics (the reference's
 //     scatter; sums in arrival order, so not bitwise reproducible);
+//   * the residual and the energy need no strain columns: a warp takes a chunk,
+//     lane (k, q) evaluates element k's strains at quadrature point q from the
+//     displacements and applies the transposed maps;
 //   * a batch of problems runs each colour of all its problems in one launch
-//     (work items = (problem, chunk) per warp), or all chunks of all
-//     problems in one launch with atomics.
+//     (work items = (problem, chunk) per CTA), or all chunks of all problems
+//     in one launch with atomics.
+// Measured on B200 (one warp taking a chunk's elements one after another with
+// stored strain matrices -> this): Jacobian and residual of a 10x10 plate
+// 169 -> 25 us, of a 400x200 plate 738 -> 307 us; residual of a 300x300 plate
+// 580 -> 95 us. The Jacobian is bound by instruction latency and shared-memory
+// wavefronts (l1tex 62 %, FP64 pipe 20 %, 15 warps an SM), the residual by
+// instruction latency (FP64 pipe 28 %).
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <thread>
 
 #include "gf_internal.h"
 
 namespace gf {
 
-constexpr int kAsmWarps = 2;     // warps (= chunks) per CTA
-constexpr int kEPW = 8;          // elements per chunk; geometry spread over 8 x 4 lanes
-constexpr int kChunkSize = kEPW;
+constexpr int kChunkSize = 8;     // elements per chunk
+constexpr int kAsmThreads = 128;  // a warp takes every fourth element
 
-struct WarpSlot {
-  double X[kEPW][12];
-  double U[kEPW][24];
-  ElemGeom g[kEPW];
-  double Bt[36][24];   // B_q[k][l] of the current element, row qk = 9q + k
-  double DBt[36][24];  // (D B_q)[k][l]
-  double E[36];
-  double S[36];
+struct ChunkSlot {
+  ElemData e[kChunkSize];
+  double U[kChunkSize][24];
+  double Re[kChunkSize][24];
+  double thick[kChunkSize];
+  Material mat[kChunkSize];
+  int4 brec[16 * kChunkSize];
 };
+
+// A block (or node) that a chunk contributes to: x = block (node), y = info,
+// (z, w) = up to eight contributions, one byte each: element of the chunk
+// * 16 + block 4a + b of the element (* 4 + node a). Info: Dirichlet rows and
+// columns (6 bits each), diagonal block, first chunk to touch it, number of
+// contributions.
+enum { kRecColShift = 6, kRecDiag = 1 << 12, kRecFirst = 1 << 13, kRecCountShift = 16 };
+
+// The records of all chunks (brec[bptr[li] ..], nrec[nptr[li] ..] for schedule
+// position li). Host threads take ranges of chunks; within a chunk a small
+// hash table finds the record of a block or node.
+static void chunk_records(const gf_mesh_desc& d, const std::vector<int32_t>& emap,
+                          const Schedule& s, const std::vector<uint8_t>& bcmask,
+                          std::vector<int4>& brec, std::vector<int32_t>& bptr,
+                          std::vector<int4>& nrec, std::vector<int32_t>& nptr) {
+  constexpr int kHash = 256;  // twice the records a chunk can have
+  const int nt = s.nchunks < 256 ? 1 : (int)std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+  struct Part {
+    std::vector<int4> brec, nrec;
+  };
+  std::vector<Part> parts(nt);
+  bptr.assign(s.nchunks + 1, 0);
+  nptr.assign(s.nchunks + 1, 0);
+  auto work = [&](int t) {
+    Part& part = parts[t];
+    const int l0 = (int)((long long)s.nchunks * t / nt), l1 = (int)((long long)s.nchunks * (t + 1) / nt);
+    part.brec.reserve((size_t)80 * (l1 - l0) + 128);
+    part.nrec.reserve((size_t)17 * (l1 - l0) + 32);
+    int16_t at[2][kHash];
+    auto add = [&](std::vector<int4>& recs, int16_t* h, size_t start, int x, int info, int code,
+                   bool first) {
+      int q = (int)(((unsigned)x * 2654435761u) >> 24);
+      while (h[q] >= 0 && recs[start + h[q]].x != x) q = (q + 1) & (kHash - 1);
+      if (h[q] < 0) {
+        h[q] = (int16_t)(recs.size() - start);
+        recs.push_back(make_int4(x, info, 0, 0));
+      }
+      int4& r = recs[start + h[q]];
+      const int n = r.y >> kRecCountShift;
+      (n < 4 ? r.z : r.w) |= (int)((unsigned)code << (8 * (n & 3)));
+      r.y += 1 << kRecCountShift;
+      if (first) r.y |= kRecFirst;
+    };
+    for (int li = l0; li < l1; li++) {
+      std::memset(at, -1, sizeof(at));
+      const size_t b0 = part.brec.size(), n0 = part.nrec.size();
+      for (int q = s.chunk_start[li]; q < s.chunk_start[li + 1]; q++) {
+        const int e = s.order[q], k = q - s.chunk_start[li];
+        for (int x = 0; x < 4; x++) {
+          const int na = d.conn[4 * e + x];
+          add(part.nrec, at[1], n0, na, bcmask[na], 4 * k + x, (s.first_touch[e] >> (16 + x)) & 1);
+          for (int y = 0; y < 4; y++)
+            add(part.brec, at[0], b0, emap[16 * e + 4 * x + y],
+                bcmask[na] | bcmask[d.conn[4 * e + y]] << kRecColShift | (x == y ? kRecDiag : 0),
+                16 * k + 4 * x + y, (s.first_touch[e] >> (4 * x + y)) & 1);
+        }
+      }
+      bptr[li + 1] = (int32_t)(part.brec.size() - b0);
+      nptr[li + 1] = (int32_t)(part.nrec.size() - n0);
+    }
+  };
+  std::vector<std::thread> th;
+  for (int t = 1; t < nt; t++) th.emplace_back(work, t);
+  work(0);
+  for (auto& x : th) x.join();
+  for (int li = 0; li < s.nchunks; li++) {
+    bptr[li + 1] += bptr[li];
+    nptr[li + 1] += nptr[li];
+  }
+  brec.reserve(bptr.back());
+  nrec.reserve(nptr.back());
+  for (auto& part : parts) {
+    brec.insert(brec.end(), part.brec.begin(), part.brec.end());
+    nrec.insert(nrec.end(), part.nrec.begin(), part.nrec.end());
+  }
+}
 
 struct AsmParams {
   const double* xpts;
   const double* vars;
-  const uint8_t* bcmask;
   const int32_t* sconn;
-  const int32_t* semap;
-  const uint32_t* sft;
   const double* sthick;
   const int32_t* smat;
   const Material* mats;
   const int32_t* chunk_start;
   const double* thick_nat;   // optional per-call thickness (natural element order)
   const int32_t* sorder;     // schedule position -> element
-  int chunk_base, chunk_end;
+  const int4* brec;          // block records of all chunks, and where a chunk's begin
+  const int32_t* bptr;
+  const int4* nrec;          // node records
+  const int32_t* nptr;
   double* values;
   double* res;
   double* energy_part;
-  int flags;
+  int chunk_base, chunk_end;
+  int flags, pad;
 };
 
 enum { MODE_JAC = 0, MODE_RES = 1, MODE_ENERGY = 2 };
 
-// Geometry of up to kEPW elements (schedule positions s0 .. s0+cnt-1).
-__device__ void batch_geometry(int s0, int cnt, WarpSlot& w, const AsmParams& P, int lane) {
-  for (int t = lane; t < cnt * 12; t += 32) {
-    const int k = t / 12, i = t % 12;
-    const int node = P.sconn[4 * (s0 + k) + i / 3];
-    w.X[k][i] = P.xpts[3 * node + i % 3];
-  }
-  for (int t = lane; t < cnt * 24; t += 32) {
-    const int k = t / 24, i = t % 24;
-    const int node = P.sconn[4 * (s0 + k) + i / 6];
-    w.U[k][i] = P.vars ? P.vars[6 * node + i % 6] : 0.0;
-  }
-  __syncwarp();
-  const int k = lane >> 2, n = lane & 3;
-  const bool on = k < cnt;
-  Material m;
-  if (on) m = P.mats[P.smat ? P.smat[s0 + k] : 0];
-  if (on) geom_normal(w.X[k], n, &w.g[k].fn[3 * n]);
-  __syncwarp();
-  if (on) {
-    geom_node(m, w.X[k], w.g[k].fn, n, w.g[k].Tn01[n], w.g[k].XTn[n], w.g[k].tcross[n]);
-    geom_quad(m, w.X[k], w.g[k].fn, n, w.g[k].T[n], w.g[k].A[n], w.g[k].Az[n],
-              w.g[k].scale[n]);
-  }
-  for (int t = lane; t < cnt * 5; t += 32) geom_tying(w.X[t / 5], w.g[t / 5].fn, t % 5, w.g[t / 5]);
-  __syncwarp();
+// c += A B over k = 4 (A row-major 8x4, B column-major 4x8, lane = 4 row + k
+// and 4 column + k); exact FP64 multiply-adds
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+// upper 8x8 tiles of a 24x24 product, one strain component of all points
+__device__ __forceinline__ void mma_step(double (&acc)[6][2], const double (&E)[3],
+                                         const double (&S)[3]) {
+  mma_f64(acc[0], E[0], S[0]);
+  mma_f64(acc[1], E[0], S[1]);
+  mma_f64(acc[2], E[0], S[2]);
+  mma_f64(acc[3], E[1], S[1]);
+  mma_f64(acc[4], E[1], S[2]);
+  mma_f64(acc[5], E[2], S[2]);
 }
 
-template <int MODE>
-__device__ void process_element(int s, int k, WarpSlot& w, const AsmParams& P, int lane,
-                                double& energy_acc) {
-  const Material m = P.mats[P.smat ? P.smat[s] : 0];
-  const double t = P.thick_nat ? P.thick_nat[P.sorder[s]] : P.sthick[s];
-  const ElemGeom& g = w.g[k];
-  if (lane < 24) {
-    double Bc[36];
-    bmat_column(g, lane, Bc);
+// K_e of one element by one warp; d holds the element's tables on entry and
+// K_e (rows of kKeStride doubles) on exit.
+__device__ __forceinline__ void element_stiffness(ElemData& d, const Material& m, double t,
+                                                  int lane) {
+  const int i = lane >> 2, q = lane & 3;
+  const Stiffness D = stiffness(m, t, d.scale[q]);
+  double acc[6][2];
 #pragma unroll
-    for (int qk = 0; qk < 36; qk++) w.Bt[qk][lane] = Bc[qk];
-    if (MODE == MODE_JAC) {
+  for (int k = 0; k < 6; k++) acc[k][0] = acc[k][1] = 0.0;
+  ColumnAt c[3];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        double Sq[9];
-        stress(m, t, g.scale[q], &Bc[9 * q], Sq);
+  for (int k = 0; k < 3; k++) c[k] = column_at(d, 8 * k + i, q);
+  double E[3], S[3];
+  // drill, then transverse shear, then (E2, E5), then (E0, E1, E3, E4)
 #pragma unroll
-        for (int kk = 0; kk < 9; kk++) w.DBt[9 * q + kk][lane] = Sq[kk];
+  for (int k = 0; k < 3; k++) E[k] = c[k].e8, S[k] = D.r * E[k];
+  mma_step(acc, E, S);
+#pragma unroll
+  for (int z = 3; z < 5; z++) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) E[k] = tying_row(d, q, z, c[k].g), S[k] = D.s * E[k];
+    mma_step(acc, E, S);
+  }
+  {
+    double E2[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) E2[k] = tying_row(d, q, 2, c[k].g);
+#pragma unroll
+    for (int k = 0; k < 3; k++) S[k] = D.a5 * E2[k] + D.b5 * c[k].e5;
+    mma_step(acc, E2, S);
+#pragma unroll
+    for (int k = 0; k < 3; k++) E[k] = c[k].e5, S[k] = D.b5 * E2[k] + D.d5 * E[k];
+    mma_step(acc, E, S);
+  }
+  {
+    double E0[3], E1[3], E3[3], E4[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      E0[k] = tying_row(d, q, 0, c[k].g);
+      E1[k] = tying_row(d, q, 1, c[k].g);
+      E3[k] = c[k].e3;
+      E4[k] = c[k].e4;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      S[k] = D.a0 * E0[k] + D.a1 * E1[k] + D.b0 * E3[k] + D.b1 * E4[k];
+    mma_step(acc, E0, S);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      S[k] = D.a1 * E0[k] + D.a0 * E1[k] + D.b1 * E3[k] + D.b0 * E4[k];
+    mma_step(acc, E1, S);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      S[k] = D.b0 * E0[k] + D.b1 * E1[k] + D.d0 * E3[k] + D.d1 * E4[k];
+    mma_step(acc, E3, S);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      S[k] = D.b1 * E0[k] + D.b0 * E1[k] + D.d1 * E3[k] + D.d0 * E4[k];
+    mma_step(acc, E4, S);
+  }
+  __syncwarp();  // the tables have been read
+  double* K = reinterpret_cast<double*>(&d);
+  int tile = 0;
+#pragma unroll
+  for (int mi = 0; mi < 3; mi++)
+#pragma unroll
+    for (int ni = mi; ni < 3; ni++, tile++) {
+      const int r = 8 * mi + i, col = 8 * ni + 2 * q;
+      *reinterpret_cast<double2*>(&K[r * kKeStride + col]) = make_double2(acc[tile][0], acc[tile][1]);
+      if (ni > mi) {
+        K[col * kKeStride + r] = acc[tile][0];
+        K[(col + 1) * kKeStride + r] = acc[tile][1];
       }
     }
-  }
-  __syncwarp();
-  const int4 cn = reinterpret_cast<const int4*>(P.sconn)[s];
-  const int nodes[4] = {cn.x, cn.y, cn.z, cn.w};
+}
+
+// Node sums of a chunk: contributions in Re (24 per element), summed in
+// element order.
+__device__ __forceinline__ void scatter_residual(const AsmParams& P, int li, const double (*Re)[24],
+                                                 int tid, int threads) {
   const bool fuse = (P.flags & GF_ASSEMBLE_FUSE_BCS) != 0;
   const bool add = (P.flags & GF_ASSEMBLE_ADD) != 0;
-  const uint32_t ft = P.sft[s];
+  const bool atomic = (P.flags & GF_ASSEMBLE_ATOMIC) != 0;
+  const int n0 = P.nptr[li], nn = 6 * (P.nptr[li + 1] - n0);
+  for (int t = tid; t < nn; t += threads) {
+    const int4 rec = __ldg(P.nrec + n0 + t / 6);
+    const int c = t % 6, n = rec.y >> kRecCountShift;
+    double v = 0.0;
+    for (int k = 0; k < n; k++) {
+      const int code = ((k < 4 ? rec.z : rec.w) >> (8 * (k & 3))) & 255;
+      v += Re[code >> 2][6 * (code & 3) + c];
+    }
+    if (fuse && ((rec.y >> c) & 1)) v = 0.0;
+    double* dst = P.res + 6 * (size_t)rec.x + c;
+    if (atomic)
+      atomicAdd(dst, v);
+    else
+      *dst = (rec.y & kRecFirst) && !add ? v : *dst + v;
+  }
+}
 
-  if (MODE == MODE_JAC) {
-    // lane (I, J): rows 3I..3I+2, columns 6J..6J+5 of K_e (one block row slice)
-    const int I = lane >> 2, J = lane & 3;
-    double acc[3][6];
+// K (and R = K_e u_e) of chunk li (in schedule order) by one CTA.
+__device__ __forceinline__ void jacobian_chunk(const AsmParams& P, int li, ChunkSlot& w) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int s0 = P.chunk_start[li], cnt = P.chunk_start[li + 1] - s0;
+  const int b0 = P.bptr[li], nblk = P.bptr[li + 1] - b0;
+  // everything the chunk reads, all loads in flight together
+  if (tid < cnt) {
+    w.thick[tid] = P.thick_nat ? P.thick_nat[P.sorder[s0 + tid]] : P.sthick[s0 + tid];
+    w.mat[tid] = P.mats[P.smat[s0 + tid]];
+  }
+  if (tid < nblk) w.brec[tid] = __ldg(P.brec + b0 + tid);
+  for (int t = tid; t < cnt * 12; t += kAsmThreads) {
+    const int k = t / 12, x = t % 12;
+    w.e[k].X[x] = P.xpts[3 * (size_t)P.sconn[4 * (s0 + k) + x / 3] + x % 3];
+  }
+  if (P.res)
+    for (int t = tid; t < cnt * 24; t += kAsmThreads) {
+      const int k = t / 24, x = t % 24;
+      w.U[k][x] = P.vars[6 * (size_t)P.sconn[4 * (s0 + k) + x / 6] + x % 6];
+    }
+  __syncthreads();
+  if (tid < 4 * cnt)
+    elem_normal(w.e[tid >> 2].X, tid & 3, &w.e[tid >> 2].fn[3 * (tid & 3)]);
+  __syncthreads();
+  {
+    // nodes on warp 0, quadrature points on warp 1
+    const int k = lane >> 2;
+    if (warp < 2 && k < cnt) elem_point(w.e[k], w.mat[k], 4 * warp + (lane & 3));
+  }
+  __syncthreads();
+  // tables: 96 translation columns, then 96 rotation columns, then bending
+  for (int t = tid; t < 96; t += kAsmThreads)
+    if (t / 12 < cnt) elem_column(w.e[t / 12], 6 * (t % 12 / 3) + t % 3);
+  for (int t = kAsmThreads - 1 - tid; t < 96; t += kAsmThreads)
+    if (t / 12 < cnt) elem_column(w.e[t / 12], 6 * (t % 12 / 3) + t % 3 + 3);
+  for (int k = warp; k < cnt; k += kAsmThreads / 32)
+    elem_bending(w.e[k], lane >> 3, (lane >> 2) & 1, lane & 3);
+  __syncthreads();
+  for (int k = warp; k < cnt; k += kAsmThreads / 32)
+    element_stiffness(w.e[k], w.mat[k], w.thick[k], lane);
+  __syncthreads();
+  const bool fuse = (P.flags & GF_ASSEMBLE_FUSE_BCS) != 0;
+  const bool add = (P.flags & GF_ASSEMBLE_ADD) != 0;
+  const bool atomic = (P.flags & GF_ASSEMBLE_ATOMIC) != 0;
+  // the colours before have scattered
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // one row (of six) of a block a thread
+  for (int t = tid; t < 6 * nblk; t += kAsmThreads) {
+    const int4 rec = w.brec[t / 6];
+    const int r = t % 6, info = rec.y, n = info >> kRecCountShift;
+    double2* dst = reinterpret_cast<double2*>(P.values + 36 * (size_t)rec.x + 6 * r);
+    const bool first = info & kRecFirst;
+    double2 o[3];
+    if (!atomic && (!first || add))
 #pragma unroll
-    for (int r = 0; r < 3; r++)
+      for (int c = 0; c < 3; c++) o[c] = dst[c];
+    else
 #pragma unroll
-      for (int c = 0; c < 6; c++) acc[r][c] = 0.0;
-#pragma unroll 4
-    for (int qk = 0; qk < 36; qk++) {
-      const double b0 = w.Bt[qk][3 * I], b1 = w.Bt[qk][3 * I + 1], b2 = w.Bt[qk][3 * I + 2];
-      const double2* dp = reinterpret_cast<const double2*>(&w.DBt[qk][6 * J]);
-      const double2 d01 = dp[0], d23 = dp[1], d45 = dp[2];
-      const double d[6] = {d01.x, d01.y, d23.x, d23.y, d45.x, d45.y};
+      for (int c = 0; c < 3; c++) o[c] = make_double2(0.0, 0.0);
+    double2 v[3] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    for (int k = 0; k < n; k++) {
+      const int code = ((k < 4 ? rec.z : rec.w) >> (8 * (k & 3))) & 255;
+      const double2* K = reinterpret_cast<const double2*>(
+          reinterpret_cast<const double*>(&w.e[code >> 4]) +
+          (6 * ((code >> 2) & 3) + r) * kKeStride + 6 * (code & 3));
 #pragma unroll
-      for (int c = 0; c < 6; c++) {
-        acc[0][c] = fma(b0, d[c], acc[0][c]);
-        acc[1][c] = fma(b1, d[c], acc[1][c]);
-        acc[2][c] = fma(b2, d[c], acc[2][c]);
+      for (int c = 0; c < 3; c++) {
+        const double2 x = K[c];
+        v[c].x += x.x;
+        v[c].y += x.y;
       }
     }
-    const int a = I >> 1, r0 = 3 * (I & 1), b = J;
-    // residual part for rows 3I..3I+2 over columns of node b
-    double rp[3];
+    if (fuse && (info & (kRecDiag - 1))) {
+      const double one = (info & kRecDiag) && first ? 1.0 : 0.0;
+      const int masked = ((info >> r) & 1) ? 63 : info >> kRecColShift;
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-      double s_ = 0.0;
-#pragma unroll
-      for (int c = 0; c < 6; c++) s_ = fma(acc[r][c], w.U[k][6 * b + c], s_);
-      rp[r] = s_;
+      for (int c = 0; c < 3; c++) {
+        if ((masked >> (2 * c)) & 1) v[c].x = r == 2 * c ? one : 0.0;
+        if ((masked >> (2 * c + 1)) & 1) v[c].y = r == 2 * c + 1 ? one : 0.0;
+      }
     }
-    if (P.values) {
-      const uint32_t bca = fuse ? P.bcmask[nodes[a]] : 0u;
-      const uint32_t bcb = fuse ? P.bcmask[nodes[b]] : 0u;
-      const bool first = (ft >> (4 * a + b)) & 1;
-      const int blk = P.semap[16 * s + 4 * a + b];
-      double* dst = P.values + 36 * (size_t)blk + 6 * r0;
-      double v[18];
 #pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-          double x = acc[r][c];
-          if (fuse && (((bca >> (r0 + r)) & 1) || ((bcb >> c) & 1)))
-            x = (a == b && r0 + r == c && first) ? 1.0 : 0.0;
-          v[6 * r + c] = x;
-        }
-      double2* d2 = reinterpret_cast<double2*>(dst);
-      if (P.flags & GF_ASSEMBLE_ATOMIC) {
-#pragma unroll
-        for (int h = 0; h < 18; h++) atomicAdd(dst + h, v[h]);
-      } else if (first && !add) {
-#pragma unroll
-        for (int h = 0; h < 9; h++) d2[h] = make_double2(v[2 * h], v[2 * h + 1]);
+    for (int c = 0; c < 3; c++) {
+      if (atomic) {
+        atomicAdd(reinterpret_cast<double*>(dst + c), v[c].x);
+        atomicAdd(reinterpret_cast<double*>(dst + c) + 1, v[c].y);
       } else {
-#pragma unroll
-        for (int h = 0; h < 9; h++) {
-          const double2 o = d2[h];
-          d2[h] = make_double2(o.x + v[2 * h], o.y + v[2 * h + 1]);
-        }
-      }
-    }
-    // R rows 3I..3I+2: sum the four column slices (lanes J = 0..3 of row group I)
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      rp[r] += __shfl_xor_sync(0xffffffffu, rp[r], 1);
-      rp[r] += __shfl_xor_sync(0xffffffffu, rp[r], 2);
-    }
-    if (P.res && J < 3) {
-      const int r = r0 + J;  // lanes J = 0,1,2 store rows r0, r0+1, r0+2
-      double val = rp[J == 0 ? 0 : (J == 1 ? 1 : 2)];
-      if (fuse && ((P.bcmask[nodes[a]] >> r) & 1)) val = 0.0;
-      double* dst = P.res + 6 * (size_t)nodes[a] + r;
-      const bool first = (ft >> (16 + a)) & 1;
-      if (P.flags & GF_ASSEMBLE_ATOMIC)
-        atomicAdd(dst, val);
-      else if (first && !add)
-        *dst = val;
-      else
-        *dst += val;
-    }
-  } else {
-    // E_q = B_q u, S_q = D E_q, R = sum_q B_q^T S_q
-    double e0 = 0.0, e1 = 0.0;
-#pragma unroll
-    for (int l = 0; l < 24; l++) {
-      e0 = fma(w.Bt[lane][l], w.U[k][l], e0);
-      if (lane < 4) e1 = fma(w.Bt[32 + lane][l], w.U[k][l], e1);
-    }
-    double* E = w.E;
-    E[lane] = e0;
-    if (lane < 4) E[32 + lane] = e1;
-    __syncwarp();
-    if (lane < 4) stress(m, t, g.scale[lane], &E[9 * lane], &w.S[9 * lane]);
-    __syncwarp();
-    if (MODE == MODE_ENERGY) {
-      if (lane == 0) {
-        double U = 0.0;
-        for (int q = 0; q < 36; q++) U += 0.5 * E[q] * w.S[q];
-        energy_acc += U;
-      }
-    } else if (lane < 24) {
-      double rj = 0.0;
-#pragma unroll
-      for (int qk = 0; qk < 36; qk++) rj = fma(w.Bt[qk][lane], w.S[qk], rj);
-      if (P.res) {
-        const int b = lane / 6, c = lane % 6;
-        if (fuse && ((P.bcmask[nodes[b]] >> c) & 1)) rj = 0.0;
-        double* dst = P.res + 6 * (size_t)nodes[b] + c;
-        const bool first = (ft >> (16 + b)) & 1;
-        if (P.flags & GF_ASSEMBLE_ATOMIC)
-          atomicAdd(dst, rj);
-        else if (first && !add)
-          *dst = rj;
-        else
-          *dst += rj;
+        dst[c] = make_double2(o[c].x + v[c].x, o[c].y + v[c].y);
       }
     }
   }
-  __syncwarp();
+  if (!P.res) return;
+  for (int t = tid; t < 24 * cnt; t += kAsmThreads) {
+    const int k = t / 24, r = t % 24;
+    const double* K = reinterpret_cast<const double*>(&w.e[k]) + r * kKeStride;
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 24; c += 2) {
+      const double2 x = *reinterpret_cast<const double2*>(K + c);
+      s = fma(x.x, w.U[k][c], s);
+      s = fma(x.y, w.U[k][c + 1], s);
+    }
+    w.Re[k][r] = s;
+  }
+  __syncthreads();
+  scatter_residual(P, li, w.Re, tid, kAsmThreads);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kAsmWarps * 32)
-    assemble_kernel(AsmParams P) {
+__global__ void __launch_bounds__(kAsmThreads, 4) jacobian_kernel(const AsmParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  WarpSlot* slots = reinterpret_cast<WarpSlot*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int li = P.chunk_base + blockIdx.x * kAsmWarps + warp;  // this warp's chunk
-  if (li >= P.chunk_end) return;
-  const int s0 = P.chunk_start[li], cnt = P.chunk_start[li + 1] - s0;
-  WarpSlot& w = slots[warp];
-  double energy_acc = 0.0;
-  batch_geometry(s0, cnt, w, P, lane);
-  for (int k = 0; k < cnt; k++) process_element<MODE>(s0 + k, k, w, P, lane, energy_acc);
-  if (MODE == MODE_ENERGY && lane == 0) P.energy_part[li] = energy_acc;
+  asm volatile("griddepcontrol.launch_dependents;");
+  jacobian_chunk(P, P.chunk_base + blockIdx.x, *reinterpret_cast<ChunkSlot*>(smem_raw));
 }
 
-// Batched form: warp w of the launch works on chunk work[w].y of problem
+// Batched form: CTA w of the launch works on chunk work[w].y of problem
 // work[w].x, whose parameters are copied to shared memory first.
-template <int MODE>
-__global__ void __launch_bounds__(kAsmWarps * 32)
-    assemble_batch_kernel(const AsmParams* __restrict__ PP, const int2* __restrict__ work,
-                          int nwork) {
+__global__ void __launch_bounds__(kAsmThreads, 4)
+    jacobian_batch_kernel(const AsmParams* __restrict__ PP, const int2* __restrict__ work) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  WarpSlot* slots = reinterpret_cast<WarpSlot*>(smem_raw);
-  __shared__ AsmParams sp[kAsmWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wi = blockIdx.x * kAsmWarps + warp;
-  if (wi >= nwork) return;
-  const int2 it = work[wi];
-  if (lane == 0) sp[warp] = PP[it.x];
+  __shared__ AsmParams sp;
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int2 it = work[blockIdx.x];
+  static_assert(sizeof(AsmParams) % 8 == 0, "copied in 8-byte words");
+  if (threadIdx.x < sizeof(AsmParams) / 8)
+    reinterpret_cast<unsigned long long*>(&sp)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long*>(PP + it.x)[threadIdx.x];
+  __syncthreads();
+  jacobian_chunk(sp, it.y, *reinterpret_cast<ChunkSlot*>(smem_raw));
+}
+
+// Residual (or energy) of a chunk by one warp, without strain columns: lane
+// (k, q) evaluates the strains of element k at quadrature point q from the
+// displacements themselves and applies the transposed maps; as node n = q of
+// the element it does the nodal work. What the four points and nodes of an
+// element exchange goes through the element's slot.
+struct ResSlot {
+  double X[12], U[24], fn[12];
+  double d[4][3];       // director displacements theta x fn of the nodes
+  double drill[4];      // nodal drill strains, then their adjoints per point
+  double V[4][15];      // per point: adjoints of u_xi, u_eta, d_xi, d_eta, d
+  double G[4][5];       // ... of the tying strains g11 g22 g12 g23 g13
+  double S8[4];         // ... of the drill strain
+  double pad;           // slots in different banks
+};
+constexpr int kResWarps = 4;  // warps (chunks) per CTA
+
+template <int MODE>
+__device__ __forceinline__ void residual_chunk(const AsmParams& P, int li, ResSlot* w,
+                                               double (*Re)[24], int lane) {
+  const int s0 = P.chunk_start[li], cnt = P.chunk_start[li + 1] - s0;
+  for (int t = lane; t < cnt * 12; t += 32) {
+    const int k = t / 12, x = t % 12;
+    w[k].X[x] = P.xpts[3 * (size_t)P.sconn[4 * (s0 + k) + x / 3] + x % 3];
+  }
+  for (int t = lane; t < cnt * 24; t += 32) {
+    const int k = t / 24, x = t % 24;
+    w[k].U[x] = P.vars[6 * (size_t)P.sconn[4 * (s0 + k) + x / 6] + x % 6];
+  }
   __syncwarp();
-  const AsmParams& P = sp[warp];
-  const int s0 = P.chunk_start[it.y], cnt = P.chunk_start[it.y + 1] - s0;
-  WarpSlot& w = slots[warp];
-  double energy_acc = 0.0;
-  batch_geometry(s0, cnt, w, P, lane);
-  for (int k = 0; k < cnt; k++) process_element<MODE>(s0 + k, k, w, P, lane, energy_acc);
+  const int k = lane >> 2, q = lane & 3, ia = q & 1, ja = q >> 1;
+  const bool on = k < cnt;
+  ResSlot& e = w[on ? k : 0];
+  if (on) {
+    double fn[3];
+    elem_normal(e.X, q, fn);
+    for (int c = 0; c < 3; c++) e.fn[3 * q + c] = fn[c];
+    cross3(&e.U[6 * q + 3], fn, e.d[q]);
+  }
+  __syncwarp();
+  PointFrame f;
+  double tc[3], sx[3], sy[3];  // this node's drill strain is sx.u_xi + sy.u_eta - tc.theta
+  Material m;
+  if (on) {
+    m = P.mats[P.smat[s0 + k]];
+    point_frame(e.X, e.fn, m, node_xi(q), node_eta(q), f);
+    const double t0[3] = {f.T[0], f.T[3], f.T[6]}, t1[3] = {f.T[1], f.T[4], f.T[7]};
+    cross3(t0, t1, tc);
+    double s = 0.0;
+    for (int c = 0; c < 3; c++) {
+      sx[c] = 0.5 * (t1[c] * f.A[0] - t0[c] * f.A[1]);
+      sy[c] = 0.5 * (t1[c] * f.A[3] - t0[c] * f.A[4]);
+      // derivatives at the node: differences along its two edges
+      const double ux = 0.5 * (e.U[12 * ja + 6 + c] - e.U[12 * ja + c]);
+      const double uy = 0.5 * (e.U[6 * ia + 12 + c] - e.U[6 * ia + c]);
+      s += sx[c] * ux + sy[c] * uy - tc[c] * e.U[6 * q + 3 + c];
+    }
+    e.drill[q] = s;
+  }
+  __syncwarp();
+  double energy = 0.0;
+  if (on) {
+    double xi, eta;
+    quad_point(q, xi, eta);
+    point_frame(e.X, e.fn, m, xi, eta, f);
+    const double t = P.thick_nat ? P.thick_nat[P.sorder[s0 + k]] : P.sthick[s0 + k];
+    const Stiffness D = stiffness(m, t, f.det);
+    double M[5][5];
+    tying_rows(f.A, M);
+    double Az[3][2];
+    point_bending(f, Az);
+    // tying strains, interpolated to the point (basis.h:314-368)
+    const double x[2] = {0.5 * (1.0 - xi), 0.5 * (1.0 + xi)};
+    const double y[2] = {0.5 * (1.0 - eta), 0.5 * (1.0 + eta)};
+    double g[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double Xc[3], Yc[3], uc[3], vc[3];
+    for (int c = 0; c < 3; c++) {
+      uc[c] = vc[c] = 0.0;
+      Xc[c] = 0.25 * (((e.X[3 + c] - e.X[c]) - e.X[6 + c]) + e.X[9 + c]);
+      Yc[c] = 0.25 * (((-e.X[c] - e.X[3 + c]) + e.X[6 + c]) + e.X[9 + c]);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {  // edges along xi (eta = -1, 1) and along eta
+      double e11 = 0.0, e13 = 0.0, e22 = 0.0, e23 = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double X = 0.5 * (e.X[6 * j + 3 + c] - e.X[6 * j + c]);
+        const double u = 0.5 * (e.U[12 * j + 6 + c] - e.U[12 * j + c]);
+        const double n = 0.5 * (e.fn[6 * j + c] + e.fn[6 * j + 3 + c]);
+        const double d = 0.5 * (e.d[2 * j][c] + e.d[2 * j + 1][c]);
+        e11 = fma(X, u, e11);
+        e13 += n * u + X * d;
+        uc[c] += 0.5 * u;
+        const double Y = 0.5 * (e.X[3 * j + 6 + c] - e.X[3 * j + c]);
+        const double v = 0.5 * (e.U[6 * j + 12 + c] - e.U[6 * j + c]);
+        const double n2 = 0.5 * (e.fn[3 * j + c] + e.fn[3 * j + 6 + c]);
+        const double d2 = 0.5 * (e.d[j][c] + e.d[j + 2][c]);
+        e22 = fma(Y, v, e22);
+        e23 += n2 * v + Y * d2;
+        vc[c] += 0.5 * v;
+      }
+      g[0] = fma(y[j], e11, g[0]);
+      g[1] = fma(x[j], e22, g[1]);
+      g[3] = fma(x[j], 0.5 * e23, g[3]);
+      g[4] = fma(y[j], 0.5 * e13, g[4]);
+    }
+    g[2] = 0.5 * (dot3(Xc, vc) + dot3(Yc, uc));
+    double E[9], S[9];
+    const int row[5] = {0, 1, 2, 6, 7};
+#pragma unroll
+    for (int r = 0; r < 5; r++)
+      E[row[r]] = M[r][0] * g[0] + M[r][1] * g[1] + M[r][2] * g[2] + M[r][3] * g[3] + M[r][4] * g[4];
+    // bending: p_j = u_xi Az_0j + u_eta Az_1j + d_xi A_0j + d_eta A_1j + d Az_2j
+    double p[2][3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double u0 = e.U[c], u1 = e.U[6 + c], u2 = e.U[12 + c], u3 = e.U[18 + c];
+      const double d0 = e.d[0][c], d1 = e.d[1][c], d2 = e.d[2][c], d3 = e.d[3][c];
+      const double ux = 0.5 * (y[0] * (u1 - u0) + y[1] * (u3 - u2));
+      const double uy = 0.5 * (x[0] * (u2 - u0) + x[1] * (u3 - u1));
+      const double dx = 0.5 * (y[0] * (d1 - d0) + y[1] * (d3 - d2));
+      const double dy = 0.5 * (x[0] * (d2 - d0) + x[1] * (d3 - d1));
+      const double d = y[0] * (x[0] * d0 + x[1] * d1) + y[1] * (x[0] * d2 + x[1] * d3);
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        p[j][c] = ux * Az[0][j] + uy * Az[1][j] + dx * f.A[j] + dy * f.A[3 + j] + d * Az[2][j];
+    }
+    const double* T = f.T;
+    E[3] = T[0] * p[0][0] + T[3] * p[0][1] + T[6] * p[0][2];
+    E[4] = T[1] * p[1][0] + T[4] * p[1][1] + T[7] * p[1][2];
+    E[5] = T[0] * p[1][0] + T[3] * p[1][1] + T[6] * p[1][2] + T[1] * p[0][0] + T[4] * p[0][1] +
+           T[7] * p[0][2];
+    E[8] = y[0] * (x[0] * e.drill[0] + x[1] * e.drill[1]) +
+           y[1] * (x[0] * e.drill[2] + x[1] * e.drill[3]);
+    S[0] = D.a0 * E[0] + D.a1 * E[1] + D.b0 * E[3] + D.b1 * E[4];
+    S[1] = D.a1 * E[0] + D.a0 * E[1] + D.b1 * E[3] + D.b0 * E[4];
+    S[2] = D.a5 * E[2] + D.b5 * E[5];
+    S[3] = D.b0 * E[0] + D.b1 * E[1] + D.d0 * E[3] + D.d1 * E[4];
+    S[4] = D.b1 * E[0] + D.b0 * E[1] + D.d1 * E[3] + D.d0 * E[4];
+    S[5] = D.b5 * E[2] + D.d5 * E[5];
+    S[6] = D.s * E[6];
+    S[7] = D.s * E[7];
+    S[8] = D.r * E[8];
+    if (MODE == MODE_ENERGY) {
+#pragma unroll
+      for (int r = 0; r < 9; r++) energy = fma(0.5 * E[r], S[r], energy);
+    } else {
+#pragma unroll
+      for (int z = 0; z < 5; z++)
+        e.G[q][z] = M[0][z] * S[0] + M[1][z] * S[1] + M[2][z] * S[2] + M[3][z] * S[6] + M[4][z] * S[7];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double p0 = T[3 * c] * S[3] + T[3 * c + 1] * S[5];
+        const double p1 = T[3 * c + 1] * S[4] + T[3 * c] * S[5];
+        e.V[q][c] = Az[0][0] * p0 + Az[0][1] * p1;
+        e.V[q][3 + c] = Az[1][0] * p0 + Az[1][1] * p1;
+        e.V[q][6 + c] = f.A[0] * p0 + f.A[1] * p1;
+        e.V[q][9 + c] = f.A[3] * p0 + f.A[4] * p1;
+        e.V[q][12 + c] = Az[2][0] * p0 + Az[2][1] * p1;
+      }
+      e.S8[q] = S[8];
+    }
+  }
+  if (MODE == MODE_ENERGY) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) energy += __shfl_xor_sync(0xffffffffu, energy, o);
+    if (lane == 0) P.energy_part[li] = energy;
+    // this launch ends after the colours before it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
+  __syncwarp();
+  // node q of element k
+  double ru[3], rd[3], dn = 0.0;
+  if (on) {
+    const double sa = node_xi(q), ta = node_eta(q);
+    double G[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // adjoints of the node's own tying points
+    for (int c = 0; c < 3; c++) ru[c] = rd[c] = 0.0;
+#pragma unroll
+    for (int z = 0; z < 4; z++) {
+      double xi, eta, N, Nx, Ne;
+      quad_point(z, xi, eta);
+      shape(q, xi, eta, N, Nx, Ne);
+      const double wx = 0.5 * (1.0 + sa * xi), wy = 0.5 * (1.0 + ta * eta);
+      G[0] = fma(wy, e.G[z][0], G[0]);
+      G[1] = fma(wx, e.G[z][1], G[1]);
+      G[2] += e.G[z][2];
+      G[3] = fma(wx, e.G[z][3], G[3]);
+      G[4] = fma(wy, e.G[z][4], G[4]);
+      dn = fma(N, e.S8[z], dn);
+      const double* V = e.V[z];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        ru[c] += Nx * V[c] + Ne * V[3 + c];
+        rd[c] += Nx * V[6 + c] + Ne * V[9 + c] + N * V[12 + c];
+      }
+    }
+    e.drill[q] = dn;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double X = 0.5 * (e.X[6 * ja + 3 + c] - e.X[6 * ja + c]);
+      const double Y = 0.5 * (e.X[3 * ia + 6 + c] - e.X[3 * ia + c]);
+      const double Xc = 0.25 * (((e.X[3 + c] - e.X[c]) - e.X[6 + c]) + e.X[9 + c]);
+      const double Yc = 0.25 * (((-e.X[c] - e.X[3 + c]) + e.X[6 + c]) + e.X[9 + c]);
+      const double n1 = 0.5 * (e.fn[6 * ja + c] + e.fn[6 * ja + 3 + c]);
+      const double n2 = 0.5 * (e.fn[3 * ia + c] + e.fn[3 * ia + 6 + c]);
+      ru[c] += 0.5 * sa * (X * G[0] + 0.5 * n1 * G[4]) + 0.5 * ta * (Y * G[1] + 0.5 * n2 * G[3]) +
+               0.125 * (sa * Yc + ta * Xc) * G[2];
+      rd[c] += 0.25 * (X * G[4] + Y * G[3]);
+    }
+  }
+  // drill adjoints of the three nodes whose strains this node's displacement
+  // enters: its own (both edges) and its neighbours along xi and eta
+  const int nx = lane ^ 1, ny = lane ^ 2;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double ax = dn * sx[c], ay = dn * sy[c];
+    const double bx = __shfl_sync(0xffffffffu, ax, nx), by = __shfl_sync(0xffffffffu, ay, ny);
+    if (on) ru[c] += 0.5 * node_xi(q) * (ax + bx) + 0.5 * node_eta(q) * (ay + by);
+  }
+  if (on) {
+    double th[3];
+    cross3(&e.fn[3 * q], rd, th);
+    for (int c = 0; c < 3; c++) {
+      Re[k][6 * q + c] = ru[c];
+      Re[k][6 * q + 3 + c] = th[c] - tc[c] * dn;
+    }
+  }
+  __syncwarp();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  scatter_residual(P, li, Re, lane, 32);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kResWarps, 3) residual_kernel(const AsmParams P) {
+  __shared__ ResSlot slots[kResWarps][kChunkSize];
+  __shared__ double Re[kResWarps][kChunkSize][24];
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int warp = threadIdx.x >> 5, li = P.chunk_base + blockIdx.x * kResWarps + warp;
+  if (li < P.chunk_end) residual_chunk<MODE>(P, li, slots[warp], Re[warp], threadIdx.x & 31);
+}
+
+// One launch of an assembly; `after` lets it start while the launch before it
+// (the colour before) still runs.
+template <class... Args>
+static cudaError_t launch_chunks(void (*kernel)(Args...), int grid, int threads, size_t smem,
+                                 bool after, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = after ? 1 : 0;
+  ::gf::count_launch();
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 __global__ void sum_kernel(const double* part, int n, double* out) {
@@ -338,53 +721,58 @@ __global__ void permute_kernel(const int32_t* perm, int nnodes, const double* in
     out[t] = in[6 * (size_t)perm[i] + k];
 }
 
-template <int MODE>
-static gf_status launch_assembly(gf_assembler* a, double* values, double* res, int flags,
-                                 cudaStream_t st, const double* thick_nat = nullptr) {
+static AsmParams asm_params(gf_assembler* a, double* values, double* res, int flags,
+                            const double* thick_nat) {
   AsmParams P;
+  std::memset(&P, 0, sizeof(P));
   P.xpts = a->d_xpts.p;
   P.vars = a->d_vars.p;
-  P.bcmask = a->d_bcmask.p;
   P.sconn = a->d_sconn.p;
-  P.semap = a->d_semap.p;
-  P.sft = a->d_sft.p;
   P.sthick = a->d_sthick.p;
   P.smat = a->d_smat.p;
   P.mats = a->d_mats.p;
   P.chunk_start = a->d_chunk_start.p;
   P.thick_nat = thick_nat;
   P.sorder = a->d_sorder.p;
+  P.brec = a->d_brec.p;
+  P.bptr = a->d_bptr.p;
+  P.nrec = a->d_nrec.p;
+  P.nptr = a->d_nptr.p;
   P.values = values;
   P.res = res;
   P.energy_part = a->d_energy_part.p;
   P.flags = flags;
-  const size_t smem = sizeof(WarpSlot) * kAsmWarps;
+  return P;
+}
+
+template <int MODE>
+static gf_status launch_assembly(gf_assembler* a, double* values, double* res, int flags,
+                                 cudaStream_t st, const double* thick_nat = nullptr) {
+  AsmParams P = asm_params(a, values, res, flags, thick_nat);
   // per device and constant, so setting it on every call is race-free
-  GF_CUDA(cudaFuncSetAttribute(assemble_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  if (MODE == MODE_JAC)
+    GF_CUDA(cudaFuncSetAttribute(jacobian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(ChunkSlot)));
   const Schedule& s = a->sched;
-  if (flags & GF_ASSEMBLE_ATOMIC) {
-    if (!(flags & GF_ASSEMBLE_ADD)) {
-      if (values) GF_CUDA(cudaMemsetAsync(values, 0, sizeof(double) * 36 * (size_t)a->pat.nnz(), st));
-      if (res) GF_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * 6 * (size_t)a->nnodes, st));
-    }
-    P.chunk_base = 0;
-    P.chunk_end = s.nchunks;
-    const int nblk = (s.nchunks + kAsmWarps - 1) / kAsmWarps;
-    if (nblk > 0) {
-      assemble_kernel<MODE><<<nblk, kAsmWarps * 32, smem, st>>>(P); ::gf::count_launch();
-      GF_CHECK_LAUNCH();
-    }
-    return GF_OK;
+  const bool atomic = (flags & GF_ASSEMBLE_ATOMIC) != 0;
+  if (atomic && !(flags & GF_ASSEMBLE_ADD)) {
+    if (values) GF_CUDA(cudaMemsetAsync(values, 0, sizeof(double) * 36 * (size_t)a->pat.nnz(), st));
+    if (res) GF_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * 6 * (size_t)a->nnodes, st));
   }
-  for (int cc = 0; cc < s.ncc; cc++) {
-    const int nch = s.cc_start[cc + 1] - s.cc_start[cc];
-    if (nch == 0) continue;
-    const int nblk = (nch + kAsmWarps - 1) / kAsmWarps;
-    P.chunk_base = s.cc_start[cc];
-    P.chunk_end = s.cc_start[cc + 1];
-    assemble_kernel<MODE><<<nblk, kAsmWarps * 32, smem, st>>>(P); ::gf::count_launch();
-    GF_CHECK_LAUNCH();
+  bool after = false;
+  for (int cc = 0; cc < (atomic ? 1 : s.ncc); cc++) {
+    const int lo = atomic ? 0 : s.cc_start[cc], hi = atomic ? s.nchunks : s.cc_start[cc + 1];
+    if (hi == lo) continue;
+    P.chunk_base = lo;
+    P.chunk_end = hi;
+    if (MODE == MODE_JAC)
+      GF_CUDA(launch_chunks(jacobian_kernel, hi - lo, kAsmThreads, sizeof(ChunkSlot), after, st,
+                            (const AsmParams)P));
+    else
+      GF_CUDA(launch_chunks(residual_kernel<MODE == MODE_JAC ? MODE_RES : MODE>,
+                            (hi - lo + kResWarps - 1) / kResWarps, 32 * kResWarps, 0, after, st,
+                            (const AsmParams)P));
+    after = true;
   }
   return GF_OK;
 }
@@ -409,25 +797,7 @@ gf_status batch_assemble(BatchAsm*& cache, const std::vector<gf_assembler*>& asm
   BatchAsm& B = *cache;
   std::vector<AsmParams> h(np);
   for (int k = 0; k < np; k++) {
-    gf_assembler* a = asms[k];
-    AsmParams& P = h[k];
-    std::memset(&P, 0, sizeof(P));
-    P.xpts = a->d_xpts.p;
-    P.vars = a->d_vars.p;
-    P.bcmask = a->d_bcmask.p;
-    P.sconn = a->d_sconn.p;
-    P.semap = a->d_semap.p;
-    P.sft = a->d_sft.p;
-    P.sthick = a->d_sthick.p;
-    P.smat = a->d_smat.p;
-    P.mats = a->d_mats.p;
-    P.chunk_start = a->d_chunk_start.p;
-    P.thick_nat = thick ? thick[k] : nullptr;
-    P.sorder = a->d_sorder.p;
-    P.values = values[k];
-    P.res = nullptr;
-    P.energy_part = a->d_energy_part.p;
-    P.flags = flags;
+    h[k] = asm_params(asms[k], values[k], nullptr, flags, thick ? thick[k] : nullptr);
   }
   const bool atomic = (flags & GF_ASSEMBLE_ATOMIC) != 0;
   if (B.flags != flags || B.host.size() != h.size() ||
@@ -464,16 +834,15 @@ gf_status batch_assemble(BatchAsm*& cache, const std::vector<gf_assembler*>& asm
   if (atomic && !(flags & GF_ASSEMBLE_ADD))
     for (int k = 0; k < np; k++)
       GF_CUDA(cudaMemsetAsync(values[k], 0, sizeof(double) * 36 * (size_t)asms[k]->pat.nnz(), st));
-  const size_t smem = sizeof(WarpSlot) * kAsmWarps;
-  GF_CUDA(cudaFuncSetAttribute(assemble_batch_kernel<MODE_JAC>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GF_CUDA(cudaFuncSetAttribute(jacobian_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(ChunkSlot)));
+  bool after = false;
   for (size_t r = 0; r + 1 < B.off.size(); r++) {
     const int nwork = B.off[r + 1] - B.off[r];
     if (nwork == 0) continue;
-    assemble_batch_kernel<MODE_JAC><<<(nwork + kAsmWarps - 1) / kAsmWarps, kAsmWarps * 32, smem,
-                                      st>>>(B.d_params.p, B.d_work.p + B.off[r], nwork);
-    ::gf::count_launch();
-    GF_CHECK_LAUNCH();
+    GF_CUDA(launch_chunks(jacobian_batch_kernel, nwork, kAsmThreads, sizeof(ChunkSlot), after, st,
+                          (const AsmParams*)B.d_params.p, (const int2*)(B.d_work.p + B.off[r])));
+    after = true;
   }
   return GF_OK;
 }
@@ -531,7 +900,8 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
     const gf_shell_data& sd = d->data[e];
     thick[e] = sd.thick;
     Material m{sd.E, sd.nu, sd.tOffset, {sd.refAxis[0], sd.refAxis[1], sd.refAxis[2]},
-               sd.has_ref_axis ? 1 : 0, 0};
+               sd.has_ref_axis ? 1 : 0, 0, 0.0, 0.0, 0.0};
+    material_constants(m);
     int found = -1;
     for (size_t k = 0; k < a->mats.size(); k++) {
       const Material& o = a->mats[k];
@@ -549,19 +919,19 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
     emat[e] = found;
   }
   const Schedule& s = a->sched;
-  std::vector<int32_t> sconn((size_t)4 * ne), semap((size_t)16 * ne), smat(ne);
-  std::vector<uint32_t> sft(ne);
+  std::vector<int32_t> sconn((size_t)4 * ne), smat(ne);
   std::vector<double> sthick(ne);
   for (int k = 0; k < ne; k++) {
     const int e = s.order[k];
     for (int x = 0; x < 4; x++) sconn[4 * k + x] = d->conn[4 * e + x];
-    for (int x = 0; x < 16; x++) semap[16 * k + x] = a->emap[16 * e + x];
-    sft[k] = s.first_touch[e];
     sthick[k] = thick[e];
     smat[k] = emat[e];
   }
   std::vector<uint8_t> bcmask(nn, 0);
   for (int i = 0; i < d->num_bcs; i++) bcmask[d->bcs[i] / 6] |= (uint8_t)(1u << (d->bcs[i] % 6));
+  std::vector<int4> brec, nrec;
+  std::vector<int32_t> bptr, nptr;
+  chunk_records(*d, a->emap, s, bcmask, brec, bptr, nrec, nptr);
   // BC entry list (solver order): rows of constrained DOFs and the matching columns
   std::vector<int32_t> ent;
   const Pattern& P = a->pat;
@@ -595,11 +965,12 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
   if (st == GF_OK) up(cudaMemset(a->d_vars.p, 0, sizeof(double) * 6 * nn));
   up(a->d_perm.upload(a->perm));
   up(a->d_bcs.upload(a->bcs));
-  up(a->d_bcmask.upload(bcmask));
   up(a->d_sconn.upload(sconn));
-  up(a->d_semap.upload(semap));
   up(a->d_smat.upload(smat));
-  up(a->d_sft.upload(sft));
+  up(a->d_brec.upload(brec));
+  up(a->d_bptr.upload(bptr));
+  up(a->d_nrec.upload(nrec));
+  up(a->d_nptr.upload(nptr));
   up(a->d_sthick.upload(sthick));
   up(a->d_sorder.upload(s.order));
   up(a->d_chunk_start.upload(s.chunk_start));

@@ -228,10 +228,11 @@ struct gf_assembler {
   // device: natural-order mesh
   gf::DevBuf<double> d_xpts, d_vars;
   gf::DevBuf<int32_t> d_perm, d_bcs;
-  gf::DevBuf<uint8_t> d_bcmask;     // per natural node, bit r = DOF r constrained
-  // device: schedule-ordered element data
-  gf::DevBuf<int32_t> d_sconn, d_semap, d_smat;
-  gf::DevBuf<uint32_t> d_sft;
+  // device: schedule-ordered element data, and the blocks and nodes that each
+  // chunk of elements contributes to
+  gf::DevBuf<int32_t> d_sconn, d_smat;
+  gf::DevBuf<int4> d_brec, d_nrec;
+  gf::DevBuf<int32_t> d_bptr, d_nptr;
   gf::DevBuf<double> d_sthick;
   gf::DevBuf<int32_t> d_sorder;     // schedule position -> element
   gf::DevBuf<int32_t> d_chunk_list, d_chunk_start;

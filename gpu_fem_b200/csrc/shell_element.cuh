@@ -4,7 +4,7 @@
 // (element, quadrature point, Jacobian column)
 // (include/shell/elem_group.h:98-303). Every map on that path is linear in
 // the DOFs, so this file writes the same strains as E_q = B_q u with the
-// 9 x 24 matrix B_q built column by column from per-element geometry that is
+// 9 x 24 matrix B_q built entry by entry from per-element tables that are
 // computed once:
 //   membrane/shear rows  e0ty = (Xd^-1 T)^T gty (Xd^-1 T) from the MITC tying
 //                        strains (include/shell/physics.h:94-209,
@@ -43,7 +43,16 @@ struct Material {
   double refAxis[3];
   int has_ref_axis;
   int pad;
+  // plane-stress stiffness (E / (1 - nu^2) times 1 and nu) and shear modulus,
+  // a2disotropicshellstress.h:12-51
+  double C0, C1, C5;
 };
+inline void material_constants(Material& m) {
+  const double D = m.E / (1.0 - m.nu * m.nu);
+  m.C0 = D;
+  m.C1 = m.nu * D;
+  m.C5 = m.E / 2.0 / (1.0 + m.nu);
+}
 
 // Node sign pattern of the tensor-product basis: node a sits at
 // (xi_a, eta_a) = (-1 + 2 (a % 2), -1 + 2 (a / 2))  (basis.h:138-142).
@@ -128,250 +137,240 @@ GF_HD void shell_transform(const Material& m, const double* Xxi, const double* n
   }
 }
 
-// Per-element geometry shared by all 24 DOF columns.
-struct ElemGeom {
-  double fn[12];        // unit node normals (ShellComputeNodeNormals, basis.h:292-311)
-  // drill strain, per node n: rows c of T_n (first two columns), rows 0/1 of
-  // Xd_n^-1 T_n, and t0 x t1 of T_n
-  double Tn01[4][6];    // [c*2 + i] = T_n[c][i], i in {0,1}
-  double XTn[4][6];     // [r*3 + j] = (Xd_n^-1 T_n)[r][j], r in {0,1}
-  double tcross[4][3];  // T_n[:,0] x T_n[:,1]
-  // quadrature points
-  double T[4][9];       // shell transform
-  double A[4][9];       // Xd^-1 T
-  double Az[4][9];      // XdinvzT = -Xd^-1 Xdz Xd^-1 T
-  double scale[4];      // detXd * weight
-  // tying points: g11/g13 at (0, -1), (0, 1); g22/g23 at (-1, 0), (1, 0); g12 at (0, 0)
-  double Xxi_t[2][3], n0_xi_t[2][3];    // at (0, eta_j)
-  double Xeta_t[2][3], n0_eta_t[2][3];  // at (xi_i, 0)
-  double Xxi_c[3], Xeta_c[3];           // at (0, 0)
-};
-
 GF_HD void quad_point(int q, double& xi, double& eta) {
   xi = (q & 1) ? kRt3 : -kRt3;
   eta = (q & 2) ? kRt3 : -kRt3;
 }
 
-// ---- geometry pieces (each independent, so warps can spread them over lanes)
-GF_HD void geom_normal(const double* X, int n, double* fn_n) {
+// Element data from which every entry of the four B_q follows with a few
+// multiplications. One element of a chunk; the assembled K_e overlays it once
+// its strains have been used (kKeStride doubles a row).
+constexpr int kKeStride = 26;  // padded rows: mirrored columns land in different banks
+struct ElemData {
+  // per DOF column l = 6a + c, independent of the quadrature point: tying
+  // strains g11, g22, g12, g23, g13 of the column (before the interpolation
+  // along the edges), the two factors of its director (or unit) vector
+  // against the columns of T, an unused entry, and its nodal drill strains
+  double tab[24][12];
+  double M[4][5][6];   // E0, E1, E2, E6, E7 from (g11, g22, g12, g23, g13)
+  double R[4][2][4][2];  // bending: (u1d Xd^-1 T + u0d XdinvzT) of [q][translation/rotation][node]
+  double T[4][6];      // first two columns of the shell frame, [q][2 c + i]
+  double scale[4];     // detXd * weight
+  // sources of the tables
+  double AA[4][10];    // Xd^-1 T (rows 0, 1) and XdinvzT (rows 0, 1, 2), first two columns
+  double Tn[4][6];     // nodal frames, first two columns
+  double XT[4][4];     // nodal Xd^-1 T, rows 0, 1, first two columns
+  double tc[4][3];     // nodal T[:,0] x T[:,1]
+  double fn[12];       // unit node normals (ShellComputeNodeNormals, basis.h:292-311)
+  double X[12];
+  double pad[10];      // elements start in different banks
+};
+static_assert(sizeof(ElemData) >= sizeof(double) * 24 * kKeStride, "K_e overlays ElemData");
+
+GF_HD void elem_normal(const double* X, int n, double* fn) {
   double v[3], xi[3], eta[3], c[3];
   interp3(X, node_xi(n), node_eta(n), v, xi, eta);
   cross3(xi, eta, c);
   const double nrm = sqrt(dot3(c, c));
-  for (int k = 0; k < 3; k++) fn_n[k] = (1.0 / nrm) * c[k];
+  for (int k = 0; k < 3; k++) fn[k] = (1.0 / nrm) * c[k];
 }
-GF_HD void geom_node(const Material& m, const double* X, const double* fn, int n,
-                     double* Tn01, double* XTn, double* tc) {
-  double v[3], xi[3], eta[3];
-  interp3(X, node_xi(n), node_eta(n), v, xi, eta);
-  const double* f = &fn[3 * n];
-  double Xd[9], Xdi[9], T[9], XT[9];
-  for (int i = 0; i < 3; i++) {
-    Xd[3 * i] = xi[i];
-    Xd[3 * i + 1] = eta[i];
-    Xd[3 * i + 2] = f[i];
-  }
-  shell_transform(m, xi, f, T);
-  inv3(Xd, Xdi);
-  mm3(Xdi, T, XT);
-  for (int c = 0; c < 3; c++) {
-    Tn01[2 * c] = T[3 * c];
-    Tn01[2 * c + 1] = T[3 * c + 1];
-  }
-  for (int j = 0; j < 6; j++) XTn[j] = XT[j];
-  const double t0[3] = {T[0], T[3], T[6]}, t1[3] = {T[1], T[4], T[7]};
-  cross3(t0, t1, tc);
-}
-GF_HD void geom_quad(const Material& m, const double* X, const double* fn, int q, double* T,
-                     double* A, double* Az, double& scale) {
-  double xi, eta;
-  quad_point(q, xi, eta);
-  double xv[3], Xxi[3], Xeta[3], n0[3], nxi[3], neta[3];
+
+// Frame of a point: Xd = [Xxi Xeta n0] with the interpolated node normals n0
+// (at a node: its own), its inverse and determinant, the shell frame T and
+// A = Xd^-1 T.
+struct PointFrame {
+  double T[9], A[9], Xdi[9], nxi[3], neta[3], det;
+};
+GF_HD void point_frame(const double* X, const double* fn, const Material& m, double xi, double eta,
+                       PointFrame& f) {
+  double xv[3], Xxi[3], Xeta[3], n0[3], Xd[9];
   interp3(X, xi, eta, xv, Xxi, Xeta);
-  interp3(fn, xi, eta, n0, nxi, neta);
-  double Xd[9], Xdz[9], Xdi[9];
+  interp3(fn, xi, eta, n0, f.nxi, f.neta);
   for (int i = 0; i < 3; i++) {
     Xd[3 * i] = Xxi[i];
     Xd[3 * i + 1] = Xeta[i];
     Xd[3 * i + 2] = n0[i];
-    Xdz[3 * i] = nxi[i];
-    Xdz[3 * i + 1] = neta[i];
-    Xdz[3 * i + 2] = 0.0;
   }
-  shell_transform(m, Xxi, n0, T);
-  const double det = inv3(Xd, Xdi);
-  mm3(Xdi, T, A);
-  double tmp[9];
-  mm3(Xdi, Xdz, tmp);
-  mm3(tmp, A, Az);
-  for (int i = 0; i < 9; i++) Az[i] = -Az[i];
-  scale = det;  // quadrature weight is 1 (quadrature.h:13-17)
+  shell_transform(m, Xxi, n0, f.T);
+  f.det = inv3(Xd, f.Xdi);
+  mm3(f.Xdi, f.T, f.A);
 }
-// k in 0..4: 0,1 -> (0, -1), (0, 1); 2,3 -> (-1, 0), (1, 0); 4 -> (0, 0)
-GF_HD void geom_tying(const double* X, const double* fn, int k, ElemGeom& g) {
-  double xi = 0.0, eta = 0.0;
-  if (k < 2) eta = k ? 1.0 : -1.0;
-  else if (k < 4) xi = (k == 3) ? 1.0 : -1.0;
-  double xv[3], Xxi[3], Xeta[3], n0[3], d1[3], d2[3];
-  interp3(X, xi, eta, xv, Xxi, Xeta);
-  interp3(fn, xi, eta, n0, d1, d2);
+// XdinvzT = -Xd^-1 Xdz Xd^-1 T, first two columns (Xdz = [n_xi n_eta 0])
+GF_HD void point_bending(const PointFrame& f, double (*Az)[2]) {
   for (int i = 0; i < 3; i++) {
-    if (k < 2) {
-      g.Xxi_t[k][i] = Xxi[i];
-      g.n0_xi_t[k][i] = n0[i];
-    } else if (k < 4) {
-      g.Xeta_t[k - 2][i] = Xeta[i];
-      g.n0_eta_t[k - 2][i] = n0[i];
-    } else {
-      g.Xxi_c[i] = Xxi[i];
-      g.Xeta_c[i] = Xeta[i];
-    }
+    const double d0 =
+        f.Xdi[3 * i] * f.nxi[0] + f.Xdi[3 * i + 1] * f.nxi[1] + f.Xdi[3 * i + 2] * f.nxi[2];
+    const double d1 =
+        f.Xdi[3 * i] * f.neta[0] + f.Xdi[3 * i + 1] * f.neta[1] + f.Xdi[3 * i + 2] * f.neta[2];
+    for (int j = 0; j < 2; j++) Az[i][j] = -(d0 * f.A[j] + d1 * f.A[3 + j]);
+  }
+}
+// E0, E1, E2, E6, E7 from the packed tying strains (g11, g22, g12, g23, g13):
+// e_ab = sum_ij A_ia G_ij A_jb, g33 = 0
+GF_HD void tying_rows(const double* A, double (*M)[5]) {
+  const int pa[5] = {0, 1, 0, 1, 0}, pb[5] = {0, 1, 1, 2, 2};
+  for (int k = 0; k < 5; k++) {
+    const int a = pa[k], b = pb[k];
+    const double w = k < 2 ? 1.0 : 2.0;
+    M[k][0] = w * (A[a] * A[b]);
+    M[k][1] = w * (A[3 + a] * A[3 + b]);
+    M[k][2] = w * (A[a] * A[3 + b] + A[3 + a] * A[b]);
+    M[k][3] = w * (A[3 + a] * A[6 + b] + A[6 + a] * A[3 + b]);
+    M[k][4] = w * (A[a] * A[6 + b] + A[6 + a] * A[b]);
   }
 }
 
-GF_HD void compute_geom(const Material& m, const double* X, ElemGeom& g) {
-  for (int n = 0; n < 4; n++) geom_normal(X, n, &g.fn[3 * n]);
-  for (int n = 0; n < 4; n++) geom_node(m, X, g.fn, n, g.Tn01[n], g.XTn[n], g.tcross[n]);
-  for (int q = 0; q < 4; q++) geom_quad(m, X, g.fn, q, g.T[q], g.A[q], g.Az[q], g.scale[q]);
-  for (int k = 0; k < 5; k++) geom_tying(X, g.fn, k, g);
-}
-
-// Column l = 6a + c of B_q for all four quadrature points: Bc[q*9 + k].
-GF_HD void bmat_column(const ElemGeom& g, int l, double* Bc) {
-  const int a = l / 6, c = l % 6;
-  const bool rot = c >= 3;
-  double v[3] = {0.0, 0.0, 0.0};  // director sensitivity e_k x fn_a (director.h:98-107)
-  if (rot) {
-    const int k = c - 3;
-    const double e[3] = {k == 0 ? 1.0 : 0.0, k == 1 ? 1.0 : 0.0, k == 2 ? 1.0 : 0.0};
-    cross3(e, &g.fn[3 * a], v);
-  }
-  // MITC tying strain sensitivities (physics.h:94-209), order
-  // g11(2) g22(2) g12(1) g23(2) g13(2)
-  double ety[9];
-  for (int j = 0; j < 2; j++) {  // points (0, eta_j)
-    const double eta = j ? 1.0 : -1.0;
-    double N, Nx, Ne;
-    shape(a, 0.0, eta, N, Nx, Ne);
-    if (!rot) {
-      ety[0 + j] = Nx * g.Xxi_t[j][c];
-      ety[7 + j] = 0.5 * g.n0_xi_t[j][c] * Nx;
-    } else {
-      ety[0 + j] = 0.0;
-      ety[7 + j] = 0.5 * dot3(g.Xxi_t[j], v) * N;
-    }
-  }
-  for (int i = 0; i < 2; i++) {  // points (xi_i, 0)
-    const double xi = i ? 1.0 : -1.0;
-    double N, Nx, Ne;
-    shape(a, xi, 0.0, N, Nx, Ne);
-    if (!rot) {
-      ety[2 + i] = Ne * g.Xeta_t[i][c];
-      ety[5 + i] = 0.5 * g.n0_eta_t[i][c] * Ne;
-    } else {
-      ety[2 + i] = 0.0;
-      ety[5 + i] = 0.5 * dot3(g.Xeta_t[i], v) * N;
-    }
-  }
-  {
-    double N, Nx, Ne;
-    shape(a, 0.0, 0.0, N, Nx, Ne);
-    ety[4] = rot ? 0.0 : 0.5 * (Nx * g.Xeta_c[c] + Ne * g.Xxi_c[c]);
-  }
-  // nodal drill strains (shell_utils.h:42-105): translations act through the
-  // in-plane displacement gradient at every node, rotations through
-  // C = I - skew(theta) at their own node.
-  double etn[4];
-  for (int n = 0; n < 4; n++) {
-    if (!rot) {
-      double N, Nx, Ne;
-      shape(a, node_xi(n), node_eta(n), N, Nx, Ne);
-      const double w0 = g.Tn01[n][2 * c], w1 = g.Tn01[n][2 * c + 1];
-      const double s0 = Nx * g.XTn[n][0] + Ne * g.XTn[n][3];
-      const double s1 = Nx * g.XTn[n][1] + Ne * g.XTn[n][4];
-      etn[n] = 0.5 * (w1 * s0 - w0 * s1);
-    } else {
-      etn[n] = (n == a) ? -g.tcross[n][c - 3] : 0.0;
-    }
-  }
-  for (int q = 0; q < 4; q++) {
-    double xi, eta;
+// Point pt of an element: nodes 0..3 (drill strain, shell_utils.h:42-105),
+// then the quadrature points 4..7.
+GF_HD void elem_point(ElemData& g, const Material& m, int pt) {
+  double xi, eta;
+  const int q = pt & 3;
+  if (pt < 4) {
+    xi = node_xi(q);
+    eta = node_eta(q);
+  } else {
     quad_point(q, xi, eta);
-    const double na0 = 0.5 * (1.0 - xi), na1 = 0.5 * (1.0 + xi);
-    const double nb0 = 0.5 * (1.0 - eta), nb1 = 0.5 * (1.0 + eta);
-    // interpTyingStrain (basis.h:314-368): packed (11, 12, 13, 22, 23, 33)
-    const double g11 = nb0 * ety[0] + nb1 * ety[1];
-    const double g22 = na0 * ety[2] + na1 * ety[3];
-    const double g12 = ety[4];
-    const double g23 = na0 * ety[5] + na1 * ety[6];
-    const double g13 = nb0 * ety[7] + nb1 * ety[8];
-    const double G[9] = {g11, g12, g13, g12, g22, g23, g13, g23, 0.0};
-    const double* A = g.A[q];
-    double H[9];  // H = G A
-    mm3(G, A, H);
-    // e_ab = sum_i A_ia H_ib
-    double e00 = 0, e11 = 0, e01 = 0, e12 = 0, e02 = 0;
-    for (int i = 0; i < 3; i++) {
-      e00 += A[3 * i] * H[3 * i];
-      e11 += A[3 * i + 1] * H[3 * i + 1];
-      e01 += A[3 * i] * H[3 * i + 1];
-      e12 += A[3 * i + 1] * H[3 * i + 2];
-      e02 += A[3 * i] * H[3 * i + 2];
-    }
-    // bending: u1x = w r^T
-    double N, Nx, Ne;
-    shape(a, xi, eta, N, Nx, Ne);
-    const double* T = g.T[q];
-    const double* Az = g.Az[q];
-    double w[2], r[2];
-    if (!rot) {
-      w[0] = T[3 * c];
-      w[1] = T[3 * c + 1];
-      r[0] = Nx * Az[0] + Ne * Az[3];
-      r[1] = Nx * Az[1] + Ne * Az[4];
-    } else {
-      w[0] = T[0] * v[0] + T[3] * v[1] + T[6] * v[2];
-      w[1] = T[1] * v[0] + T[4] * v[1] + T[7] * v[2];
-      r[0] = Nx * A[0] + Ne * A[3] + N * Az[6];
-      r[1] = Nx * A[1] + Ne * A[4] + N * Az[7];
-    }
-    double et = 0.0;
-    for (int n = 0; n < 4; n++) {
-      double Nn, dx, de;
-      shape(n, xi, eta, Nn, dx, de);
-      et += Nn * etn[n];
-    }
-    double* E = &Bc[9 * q];
-    E[0] = e00;
-    E[1] = e11;
-    E[2] = 2.0 * e01;
-    E[3] = w[0] * r[0];
-    E[4] = w[1] * r[1];
-    E[5] = w[0] * r[1] + w[1] * r[0];
-    E[6] = 2.0 * e12;
-    E[7] = 2.0 * e02;
-    E[8] = et;
+  }
+  PointFrame f;
+  point_frame(g.X, g.fn, m, xi, eta, f);
+  double* T = pt < 4 ? g.Tn[q] : g.T[q];
+  for (int c = 0; c < 3; c++) {
+    T[2 * c] = f.T[3 * c];
+    T[2 * c + 1] = f.T[3 * c + 1];
+  }
+  if (pt < 4) {
+    g.XT[q][0] = f.A[0];
+    g.XT[q][1] = f.A[1];
+    g.XT[q][2] = f.A[3];
+    g.XT[q][3] = f.A[4];
+    const double t0[3] = {f.T[0], f.T[3], f.T[6]}, t1[3] = {f.T[1], f.T[4], f.T[7]};
+    cross3(t0, t1, g.tc[q]);
+    return;
+  }
+  double Az[3][2], M[5][5];
+  point_bending(f, Az);
+  for (int j = 0; j < 2; j++) {
+    g.AA[q][j] = f.A[j];
+    g.AA[q][2 + j] = f.A[3 + j];
+    for (int i = 0; i < 3; i++) g.AA[q][4 + 2 * i + j] = Az[i][j];
+  }
+  g.scale[q] = f.det;  // quadrature weight is 1 (quadrature.h:13-17)
+  tying_rows(f.A, M);
+  for (int k = 0; k < 5; k++) {
+    for (int z = 0; z < 5; z++) g.M[q][k][z] = M[k][z];
+    g.M[q][k][5] = 0.0;
   }
 }
 
-// S = D E for the isotropic shell (a2disotropicshellstress.h:12-51), scaled.
-GF_HD void stress(const Material& m, double t, double s, const double* E, double* S) {
-  const double Dm = m.E / (1.0 - m.nu * m.nu);
-  const double C0 = Dm, C1 = m.nu * Dm, C5 = m.E / 2.0 / (1.0 + m.nu);
+// Table of DOF column l = 6a + c (MITC tying strain sensitivities,
+// physics.h:94-209, and nodal drill strains, shell_utils.h:42-105). A node's
+// shape functions vanish on the edges it does not lie on, so each tying
+// strain of a column comes from the one point of its node's edge.
+GF_HD void elem_column(ElemData& g, int l) {
+  const int a = l / 6, c = l % 6, ia = a & 1, ja = a >> 1;
+  const double sa = node_xi(a), ta = node_eta(a);
+  const double* f = &g.fn[3 * a];
+  const double *X0 = &g.X[6 * ja], *X1 = X0 + 3;           // the node's edge along xi
+  const double *Y0 = &g.X[3 * ia], *Y1 = Y0 + 6;           // ... along eta
+  double* t = g.tab[l];
+  t[7] = 0.0;
+  if (c < 3) {
+    t[0] = 0.5 * sa * (0.5 * (X1[c] - X0[c]));
+    t[1] = 0.5 * ta * (0.5 * (Y1[c] - Y0[c]));
+    // centre tangents, summed over the nodes in order like every interpolation
+    const double Xc = 0.25 * (((g.X[3 + c] - g.X[c]) - g.X[6 + c]) + g.X[9 + c]);
+    const double Yc = 0.25 * (((-g.X[c] - g.X[3 + c]) + g.X[6 + c]) + g.X[9 + c]);
+    t[2] = 0.5 * (0.25 * sa * Yc + 0.25 * ta * Xc);
+    t[3] = 0.25 * ta * (0.5 * (g.fn[3 * ia + c] + g.fn[3 * ia + 6 + c]));
+    t[4] = 0.25 * sa * (0.5 * (g.fn[6 * ja + c] + g.fn[6 * ja + 3 + c]));
+    t[5] = 1.0;
+    t[6] = 0.0;
+    for (int n = 0; n < 4; n++) {
+      const double Nx = (n >> 1) == ja ? 0.5 * sa : 0.0, Ne = (n & 1) == ia ? 0.5 * ta : 0.0;
+      const double s0 = Nx * g.XT[n][0] + Ne * g.XT[n][2];
+      const double s1 = Nx * g.XT[n][1] + Ne * g.XT[n][3];
+      t[8 + n] = 0.5 * (g.Tn[n][2 * c + 1] * s0 - g.Tn[n][2 * c] * s1);
+    }
+  } else {
+    // X . (e_k x f) = (f x X)_k: director sensitivity (director.h:98-107)
+    const int k = c - 3, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    t[0] = t[1] = t[2] = 0.0;
+    t[3] = 0.125 * (f[k1] * (Y1[k2] - Y0[k2]) - f[k2] * (Y1[k1] - Y0[k1]));
+    t[4] = 0.125 * (f[k1] * (X1[k2] - X0[k2]) - f[k2] * (X1[k1] - X0[k1]));
+    t[5] = f[k1];
+    t[6] = f[k2];
+    for (int n = 0; n < 4; n++) t[8 + n] = n == a ? -g.tc[a][k] : 0.0;
+  }
+}
+// entry R[q][rot][a]: bending factors of node a's translations / rotations
+// (basis.h:452-493)
+GF_HD void elem_bending(ElemData& g, int q, int rot, int a) {
+  double xi, eta, N, Nx, Ne;
+  quad_point(q, xi, eta);
+  shape(a, xi, eta, N, Nx, Ne);
+  const double* A = g.AA[q];
+  for (int j = 0; j < 2; j++)
+    g.R[q][rot][a][j] =
+        rot ? Nx * A[j] + Ne * A[2 + j] + N * A[8 + j] : Nx * A[4 + j] + Ne * A[6 + j];
+}
+
+// What a thread keeps of column l at quadrature point q: the interpolated
+// tying strains g[5] and the bending and drill strains.
+struct ColumnAt {
+  double g[5], e3, e4, e5, e8;
+};
+GF_HD ColumnAt column_at(const ElemData& d, int l, int q) {
+  const int a = l / 6, c = l % 6;
+  double xi, eta;
+  quad_point(q, xi, eta);
+  const double na = 0.5 * (1.0 + node_xi(a) * xi), nb = 0.5 * (1.0 + node_eta(a) * eta);
+  const double* t = d.tab[l];
+  ColumnAt o;
+  // interpTyingStrain (basis.h:314-368)
+  o.g[0] = nb * t[0];
+  o.g[1] = na * t[1];
+  o.g[2] = t[2];
+  o.g[3] = na * t[3];
+  o.g[4] = nb * t[4];
+  // w = T^T (e_c) for translations, T^T (e_k x f) = (f x T)_k for rotations
+  const int k = c - 3;
+  const int i1 = c < 3 ? c : (k == 0 ? 2 : k - 1), i2 = c < 3 ? c : (k == 2 ? 0 : k + 1);
+  const double* T = d.T[q];
+  const double w0 = t[5] * T[2 * i1] - t[6] * T[2 * i2];
+  const double w1 = t[5] * T[2 * i1 + 1] - t[6] * T[2 * i2 + 1];
+  const double* r = d.R[q][c < 3 ? 0 : 1][a];
+  o.e3 = w0 * r[0];
+  o.e4 = w1 * r[1];
+  o.e5 = w0 * r[1] + w1 * r[0];
+  const double x0 = 0.5 * (1.0 - xi), x1 = 0.5 * (1.0 + xi);
+  const double y0 = 0.5 * (1.0 - eta), y1 = 0.5 * (1.0 + eta);
+  o.e8 = x0 * y0 * t[8] + x1 * y0 * t[9] + x0 * y1 * t[10] + x1 * y1 * t[11];
+  return o;
+}
+// row k (E0, E1, E2, E6, E7) of the membrane / transverse shear strains
+GF_HD double tying_row(const ElemData& d, int q, int k, const double* g) {
+  const double* m = d.M[q][k];
+  return m[0] * g[0] + m[1] * g[1] + m[2] * g[2] + m[3] * g[3] + m[4] * g[4];
+}
+
+// Isotropic shell stiffnesses at a point, times the point's weight
+// (a2disotropicshellstress.h:12-51): S = D E with the membrane-bending
+// blocks a, b, d times (c0, c1; c1, c0) and c5, shear s, drill r.
+struct Stiffness {
+  double a0, a1, a5, b0, b1, b5, d0, d1, d5, s, r;
+};
+GF_HD Stiffness stiffness(const Material& m, double t, double w) {
+  const double C0 = m.C0, C1 = m.C1, C5 = m.C5;
   const double to = m.tOffset;
-  const double a = s * t, b = -s * t * t * to, d = s * (t * t * t / 12.0 + t * t * t * to * to);
-  const double m0 = C0 * E[0] + C1 * E[1], m1 = C1 * E[0] + C0 * E[1], m2 = C5 * E[2];
-  const double k0 = C0 * E[3] + C1 * E[4], k1 = C1 * E[3] + C0 * E[4], k2 = C5 * E[5];
-  S[0] = a * m0 + b * k0;
-  S[1] = a * m1 + b * k1;
-  S[2] = a * m2 + b * k2;
-  S[3] = b * m0 + d * k0;
-  S[4] = b * m1 + d * k1;
-  S[5] = b * m2 + d * k2;
+  const double a = w * t, b = -w * t * t * to, d = w * (t * t * t / 12.0 + t * t * t * to * to);
+  Stiffness o;
+  o.a0 = a * C0, o.a1 = a * C1, o.a5 = a * C5;
+  o.b0 = b * C0, o.b1 = b * C1, o.b5 = b * C5;
+  o.d0 = d * C0, o.d1 = d * C1, o.d5 = d * C5;
   const double As = kShear * t * C5;
-  S[6] = s * As * E[6];
-  S[7] = s * As * E[7];
-  S[8] = s * kDrill * As * E[8];
+  o.s = w * As;
+  o.r = w * kDrill * As;
+  return o;
 }
 
 }  // namespace gf
