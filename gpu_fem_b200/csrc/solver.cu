@@ -206,52 +206,44 @@ __global__ void bspmv_kernel(int nrows, const int32_t* __restrict__ row_prob,
 }
 
 // ----------------------------------------------------- block ILU factorization
-__device__ void inv6_warp(double* M, double* Inv, int lane, SweepCtl* ctl, int row) {
-  for (int t = lane; t < 36; t += 32) Inv[t] = (t / 6 == t % 6) ? 1.0 : 0.0;
-  __syncwarp();
+// Inverse of a 6x6 block by Gauss-Jordan elimination with row pivoting, in
+// registers: lane j < 6 holds column j of the block, lane 6 + j column j of
+// the identity (and of the inverse on return); the other lanes repeat them.
+// Column c is broadcast once a step, every lane picks the pivot for itself.
+__device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
+  bool ok = true;
+#pragma unroll
   for (int c = 0; c < 6; c++) {
+    double f[6];
+#pragma unroll
+    for (int r = 0; r < 6; r++) f[r] = __shfl_sync(0xffffffffu, m[r], c);
     int p = c;
-    double best = fabs(M[6 * c + c]);
+    double best = fabs(f[c]);
+#pragma unroll
     for (int r = c + 1; r < 6; r++) {
-      const double v = fabs(M[6 * r + c]);
+      const double v = fabs(f[r]);
       if (v > best) {
         best = v;
         p = r;
       }
     }
-    if (!(best > 0.0) || !isfinite(best)) {
-      if (lane == 0) {
-        atomicOr(&ctl->status, ST_ZERO_PIVOT);
-        atomicCAS(&ctl->pivot, 0, row + 1);
+    ok = ok && best > 0.0 && isfinite(best);
+#pragma unroll
+    for (int r = c + 1; r < 6; r++)
+      if (p == r) {
+        double t = m[c];
+        m[c] = m[r];
+        m[r] = t;
+        t = f[c];
+        f[c] = f[r];
+        f[r] = t;
       }
-    }
-    __syncwarp();
-    if (p != c && lane < 12) {
-      double* src = lane < 6 ? M : Inv;
-      const int k = lane % 6;
-      const double t0 = src[6 * p + k];
-      src[6 * p + k] = src[6 * c + k];
-      src[6 * c + k] = t0;
-    }
-    __syncwarp();
-    const double piv = 1.0 / M[6 * c + c];
-    __syncwarp();
-    if (lane < 12) {
-      double* dst = lane < 6 ? M : Inv;
-      dst[6 * c + lane % 6] *= piv;
-    }
-    __syncwarp();
-    double f[6];
-    for (int r = 0; r < 6; r++) f[r] = M[6 * r + c];
-    __syncwarp();
-    for (int t = lane; t < 72; t += 32) {
-      const int half = t / 36, rr = (t % 36) / 6, k = t % 6;
-      if (rr == c) continue;
-      double* dst = half ? Inv : M;
-      dst[6 * rr + k] -= f[rr] * dst[6 * c + k];
-    }
-    __syncwarp();
+    m[c] *= 1.0 / f[c];
+#pragma unroll
+    for (int r = 0; r < 6; r++)
+      if (r != c) m[r] = fma(-f[r], m[c], m[r]);
   }
+  return ok;
 }
 
 // IKJ block ILU on each problem's ILU pattern (FP64, in place): lower blocks
@@ -259,33 +251,38 @@ __device__ void inv6_warp(double* M, double* Inv, int lane, SweepCtl* ctl, int r
 // One warp factors one row. The row's values are staged in the warp's slice
 // of shared memory (rows up to kFacVals blocks; longer rows are updated in
 // global memory), so the read-modify-writes of the sequential steps cost a
-// shared-memory latency, and the row is written back whole when it is final.
-// Within a row the steps k (its lower blocks, ascending) are sequential; a
-// step's updates A_ij -= L_ik U_kj over j in U(k) are spread over the lanes
-// (lane = block slot b < 5, column c < 6; 2 slot batches in flight). The
-// column lists and U_kj values of a step's first batch (final rows in
-// global memory) are loaded together with U_kk^{-1}. Each row's column
-// indices are staged for the searches j -> slot.
+// shared-memory latency. Within a row the steps k (its lower blocks) are
+// sequential; a step's updates A_ij -= L_ik U_kj over j in U(k) are spread
+// over the lanes (lane = block slot b < 5, column c < 6).
 //
 // Scheduling is dataflow, not level-synchronous: the warps of the CTAs a
 // problem is given take its rows in factorization order (ascending lower
 // level) from a per-problem counter, and step k of row i waits only until
 // row k is final (its flag done[k] equals the launch's epoch, stored with
-// release after all of row k's values). Rows of later levels therefore run
+// release after row k's upper part). Rows of later levels therefore run
 // while the rows they do not read are still being factored, and a row's
 // early steps overlap the end of the rows it reads last. Every row that a
 // warp waits for has a lower level, so it was taken earlier by a warp that
 // is running; the waits end whatever the CTAs' residency. Each wait is still
 // bounded: the first that runs out sets ST_TIMEOUT, which ends the others.
+//
+// The factorization lasts levels x the chain from one row's flag to the next
+// row's: the flag becomes visible, U(k) and U_kk^{-1} arrive, one step, the
+// inverse, the stores. Everything else is kept off that chain: the extents
+// and columns of U(k) and the slots they update come from the pattern alone
+// and are looked up a step ahead, before the wait; the wait polls one
+// acquiring load (the limit is checked every 64th time); the inverse stays in
+// registers; and the flag follows the upper part of the row at once (nobody
+// reads the lower part in this launch), released by one lane.
 constexpr int kFacWarps = 8;
 constexpr int kFacRow = 256;    // row blocks whose columns are staged in shared memory
 constexpr int kFacVals = 80;    // row blocks whose values are staged in shared memory
+constexpr int kFacSteps = 128;  // steps whose extent of U(k) is staged
 constexpr int kFacPass = 6;     // passes of 5 U(k) blocks loaded at the start of a step
 constexpr int kFacBatch = 2;    // passes of 5 blocks in flight per lane beyond those
 constexpr int kFacMap = 1024;   // column span of a row whose column -> slot map is kept
-// per warp: values, L_ik, the diagonal block and its inverse, columns, map
-// and the row's step order
-constexpr size_t kFacWarpSmem = sizeof(double) * (36 * kFacVals + 3 * 36) +
+// per warp: values, L_ik, U(k) extents, columns, map and the row's step order
+constexpr size_t kFacWarpSmem = sizeof(double) * (36 * kFacVals + 36) + sizeof(int2) * kFacSteps +
                                 sizeof(int32_t) * kFacRow + sizeof(int16_t) * (kFacMap + kFacRow);
 constexpr size_t kFacSmem = kFacWarps * kFacWarpSmem;
 
@@ -306,29 +303,30 @@ __device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_release_gpu(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// Waits (bounded) until *flag == want, then acquires what its writer
-// released. False when the bound ran out (ST_TIMEOUT set here) or another
-// wait already ran out.
-__device__ bool wait_flag(const int* flag, int want, unsigned long long limit, SweepCtl* ctl) {
-  if (ld_relaxed_gpu(flag) == want) {
-    fence_acq_rel_gpu();
-    return true;
-  }
-  const unsigned long long t0 = gtimer();
-  while (true) {
-    if (ld_relaxed_gpu(flag) == want) {
-      fence_acq_rel_gpu();
-      return true;
-    }
-    if (ld_relaxed_gpu(&ctl->status) & ST_TIMEOUT) return false;
-    if (gtimer() - t0 > limit) {
-      atomicOr(&ctl->status, ST_TIMEOUT);
-      return false;
+// Waits (bounded) until *flag == want and acquires what its writer released.
+// False when the bound ran out (ST_TIMEOUT set here) or another wait already
+// ran out.
+__device__ __forceinline__ bool wait_flag(const int* flag, int want, unsigned long long limit,
+                                          SweepCtl* ctl) {
+  unsigned long long t0 = 0;
+  for (unsigned n = 0;; n++) {
+    if (ld_acquire_gpu(flag) == want) return true;
+    if ((n & 63u) == 63u) {
+      if (t0 == 0) t0 = gtimer();
+      if (ld_relaxed_gpu(&ctl->status) & ST_TIMEOUT) return false;
+      if (gtimer() - t0 > limit) {
+        atomicOr(&ctl->status, ST_TIMEOUT);
+        return false;
+      }
     }
   }
 }
@@ -344,9 +342,8 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
   unsigned char* ws = fsm + (size_t)warp * kFacWarpSmem;
   double* sR = reinterpret_cast<double*>(ws);  // staged row values
   double* Lb = sR + 36 * kFacVals;             // L_ik of the current step
-  double* sM = Lb + 36;                        // diagonal block (pivoting copy)
-  double* sI = sM + 36;                        // its inverse
-  int32_t* sC = reinterpret_cast<int32_t*>(sI + 36);
+  int2* sU = reinterpret_cast<int2*>(Lb + 36);  // step t -> blocks of U(k)
+  int32_t* sC = reinterpret_cast<int32_t*>(sU + kFacSteps);
   int16_t* sMap = reinterpret_cast<int16_t*>(sC + kFacRow);  // column - base -> slot - r0, or -1
   int16_t* sOrd = sMap + kFacMap;                              // step t -> slot - r0
   for (int t = lane; t < kFacMap; t += 32) sMap[t] = -1;
@@ -373,6 +370,11 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
     const bool vstaged = len <= kFacVals;
     const int32_t* rc = cstaged ? sC - r0 : cols;  // rc[kp] = column of slot kp
     double* R = vstaged ? sR - 36 * (size_t)r0 : LU;  // R[36 kp + e] = entry e of slot kp
+    // extent of U(k) for the steps, staged ahead (columns read from global)
+    for (int t = lane; t < min(di - r0, kFacSteps); t += 32) {
+      const int k = cols[d.pord[r0 + t]];
+      sU[t] = make_int2(diag[k] + 1, rowp[k + 1]);
+    }
     if (cstaged) {
       for (int t = lane; t < len; t += 32) sC[t] = cols[r0 + t];
       for (int t = lane; t < di - r0; t += 32) sOrd[t] = (int16_t)(d.pord[r0 + t] - r0);
@@ -386,39 +388,75 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
     if (mapped)
       for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = (int16_t)t;
     if (vstaged) {
-      // eight loads in flight per lane
-      const double* src = LU + 36 * (size_t)r0;
-      const int nv = 36 * len;
-      for (int t0 = 0; t0 < nv; t0 += 256) {
-        double v[8];
+      // four 16-byte loads in flight per lane
+      const double2* src = reinterpret_cast<const double2*>(LU + 36 * (size_t)r0);
+      double2* dst = reinterpret_cast<double2*>(sR);
+      const int nv = 18 * len;
+      for (int t0 = 0; t0 < nv; t0 += 128) {
+        double2 v[4];
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
+        for (int q = 0; q < 4; q++) {
           const int t = t0 + 32 * q + lane;
-          v[q] = t < nv ? src[t] : 0.0;
+          v[q] = t < nv ? src[t] : make_double2(0.0, 0.0);
         }
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
+        for (int q = 0; q < 4; q++) {
           const int t = t0 + 32 * q + lane;
-          if (t < nv) sR[t] = v[q];
+          if (t < nv) dst[t] = v[q];
         }
       }
     }
     __syncwarp();
+    auto extent = [&](int st, int kp) {
+      if (st - r0 < kFacSteps) return sU[st - r0];
+      const int k = rc[kp];
+      return make_int2(diag[k] + 1, rowp[k + 1]);
+    };
+    // slot of the row that column j of U(k) updates, or -1 (j < 0: none)
+    auto target = [&](int j, int kp) {
+      if (j < 0) return -1;
+      if (!mapped) return find_col(rc, kp + 1, r1, j);
+      const int off = j - cbase;
+      const int m = off < span ? sMap[off] : -1;
+      return m >= 0 ? r0 + m : -1;
+    };
+    // this step's slot, extent of U(k) and targets of its first blocks
+    int kp = r0, tp[kFacPass];
+    int2 ext = make_int2(0, 0);
+    if (r0 < di) {
+      kp = step_slot(r0);
+      ext = extent(r0, kp);
+#pragma unroll
+      for (int q = 0; q < kFacPass; q++) {
+        const int jp = ext.x + 5 * q + b;
+        tp[q] = target(lane < 30 && jp < ext.y ? cols[jp] : -1, kp);
+      }
+    }
     unsigned ready = 0;  // bit s: the row of step (window start + s) is final
     for (int st = r0; st < di; st++) {
-      const int kp = step_slot(st);
       const int s = (st - r0) & 31;
       if (s == 0) {
         // the flags of the next 32 steps, one per lane; a lane that sees
         // its row final acquires it for the warp (the warp barrier below
         // orders that acquire before every lane's later loads)
         const int q = st + lane;
-        const int f = q < di ? (ld_relaxed_gpu(done + rc[step_slot(q)]) == epoch) : 1;
-        fence_acq_rel_gpu();
+        const int f = q < di ? (ld_acquire_gpu(done + rc[step_slot(q)]) == epoch) : 1;
         ready = __ballot_sync(0xffffffffu, f);
         __syncwarp();
       }
-      const int k = rc[kp];
+      const int k = rc[kp], u0 = ext.x, u1 = ext.y;
+      // the next step's columns, in flight during this one
+      int kpn = kp, jn[kFacPass];
+      int2 extn = make_int2(0, 0);
+      if (st + 1 < di) {
+        kpn = step_slot(st + 1);
+        extn = extent(st + 1, kpn);
+      }
+#pragma unroll
+      for (int q = 0; q < kFacPass; q++) {
+        const int jp = extn.x + 5 * q + b;
+        jn[q] = lane < 30 && jp < extn.y ? __ldg(cols + jp) : -1;
+      }
       if (!((ready >> s) & 1u)) {
         int ok = lane == 0 ? (int)wait_flag(done + k, epoch, wlim, ctl) : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -428,33 +466,27 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
           break;
         }
       }
-      const int u0 = diag[k] + 1, u1 = rowp[k + 1];
-      // loads that do not depend on this row's earlier steps, all in flight
-      // together: the first kFacPass x 5 blocks of U(k) (columns and values)
-      // and U_kk^{-1}
-      int jc[kFacPass];
-      double u[kFacPass][6];
+      // U_kk^{-1} and the first kFacPass x 5 blocks of U(k), all in flight
+      const double* Ukk = LU + 36 * (size_t)(u0 - 1);
+      const int r = lane / 6, cc = lane % 6, r2 = (lane + 32) / 6, c2 = (lane + 32) % 6;
+      double uk[6], uk2[6], u[kFacPass][6];
+#pragma unroll
+      for (int m = 0; m < 6; m++) uk[m] = __ldcg(Ukk + 6 * m + cc);
+#pragma unroll
+      for (int m = 0; m < 6; m++) uk2[m] = lane < 4 ? __ldcg(Ukk + 6 * m + c2) : 0.0;
 #pragma unroll
       for (int q = 0; q < kFacPass; q++) {
-        const int jp = u0 + 5 * q + b;
-        const bool in = lane < 30 && jp < u1;
-        jc[q] = in ? cols[jp] : -1;
+        const double* src = LU + 36 * (size_t)(u0 + 5 * q + b) + c;
 #pragma unroll
-        for (int m = 0; m < 6; m++) u[q][m] = in ? LU[36 * (size_t)jp + 6 * m + c] : 0.0;
+        for (int m = 0; m < 6; m++) u[q][m] = tp[q] >= 0 ? __ldcg(src + 6 * m) : 0.0;
       }
-      const double* Ukk = LU + 36 * (size_t)diag[k];
       double* Aik = R + 36 * (size_t)kp;
       double s0 = 0.0, s1 = 0.0;
-      {
-        const int r = lane / 6, cc = lane % 6;
 #pragma unroll
-        for (int m = 0; m < 6; m++) s0 = fma(Aik[6 * r + m], Ukk[6 * m + cc], s0);
-        if (lane < 4) {
-          const int r2 = (lane + 32) / 6, c2 = (lane + 32) % 6;
+      for (int m = 0; m < 6; m++) s0 = fma(Aik[6 * r + m], uk[m], s0);
+      if (lane < 4)
 #pragma unroll
-          for (int m = 0; m < 6; m++) s1 = fma(Aik[6 * r2 + m], Ukk[6 * m + c2], s1);
-        }
-      }
+        for (int m = 0; m < 6; m++) s1 = fma(Aik[6 * r2 + m], uk2[m], s1);
       __syncwarp();
       Lb[lane] = s0;
       Aik[lane] = s0;
@@ -464,36 +496,28 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
       }
       __syncwarp();
       {
-        // targets of the prefetched blocks (distinct slots of this row), then
-        // all their reads before any write
-        int tp[kFacPass];
-#pragma unroll
-        for (int q = 0; q < kFacPass; q++) {
-          if (mapped) {
-            const int off = jc[q] - cbase;
-            const int m = (jc[q] >= 0 && off < span) ? sMap[off] : -1;
-            tp[q] = m >= 0 ? r0 + m : -1;
-          } else {
-            tp[q] = jc[q] >= 0 ? find_col(rc, kp + 1, r1, jc[q]) : -1;
-          }
-        }
+        // the targets are distinct slots of this row: all their reads before
+        // any write
         double lb[36];  // L_ik in registers for the updates
 #pragma unroll
-        for (int t = 0; t < 36; t++) lb[t] = Lb[t];
+        for (int t = 0; t < 36; t += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(Lb + t);
+          lb[t] = v.x, lb[t + 1] = v.y;
+        }
         double a[kFacPass][6];
 #pragma unroll
         for (int q = 0; q < kFacPass; q++)
 #pragma unroll
-          for (int r = 0; r < 6; r++) a[q][r] = tp[q] >= 0 ? R[36 * (size_t)tp[q] + 6 * r + c] : 0.0;
+          for (int e = 0; e < 6; e++) a[q][e] = tp[q] >= 0 ? R[36 * (size_t)tp[q] + 6 * e + c] : 0.0;
 #pragma unroll
         for (int q = 0; q < kFacPass; q++)
           if (tp[q] >= 0) {
 #pragma unroll
-            for (int r = 0; r < 6; r++) {
+            for (int e = 0; e < 6; e++) {
               double sacc = 0.0;
 #pragma unroll
-              for (int m = 0; m < 6; m++) sacc = fma(lb[6 * r + m], u[q][m], sacc);
-              R[36 * (size_t)tp[q] + 6 * r + c] = a[q][r] - sacc;
+              for (int m = 0; m < 6; m++) sacc = fma(lb[6 * e + m], u[q][m], sacc);
+              R[36 * (size_t)tp[q] + 6 * e + c] = a[q][e] - sacc;
             }
           }
       }
@@ -505,65 +529,68 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
         for (int q = 0; q < kFacBatch; q++) {
           const int jp = jb + 5 * q + b;
           const bool in = lane < 30 && jp < u1;
-          jt[q] = in ? cols[jp] : -1;
+          jt[q] = in ? __ldg(cols + jp) : -1;
 #pragma unroll
-          for (int m = 0; m < 6; m++) v[q][m] = in ? LU[36 * (size_t)jp + 6 * m + c] : 0.0;
+          for (int m = 0; m < 6; m++) v[q][m] = in ? __ldcg(LU + 36 * (size_t)jp + 6 * m + c) : 0.0;
         }
-        int tp[kFacBatch];
+        int tq[kFacBatch];
 #pragma unroll
-        for (int q = 0; q < kFacBatch; q++) {
-          if (mapped) {
-            const int off = jt[q] - cbase;
-            const int m = (jt[q] >= 0 && off < span) ? sMap[off] : -1;
-            tp[q] = m >= 0 ? r0 + m : -1;
-          } else {
-            tp[q] = jt[q] >= 0 ? find_col(rc, kp + 1, r1, jt[q]) : -1;
-          }
-        }
+        for (int q = 0; q < kFacBatch; q++) tq[q] = target(jt[q], kp);
         double a[kFacBatch][6];
 #pragma unroll
         for (int q = 0; q < kFacBatch; q++)
 #pragma unroll
-          for (int r = 0; r < 6; r++) a[q][r] = tp[q] >= 0 ? R[36 * (size_t)tp[q] + 6 * r + c] : 0.0;
+          for (int e = 0; e < 6; e++) a[q][e] = tq[q] >= 0 ? R[36 * (size_t)tq[q] + 6 * e + c] : 0.0;
 #pragma unroll
         for (int q = 0; q < kFacBatch; q++)
-          if (tp[q] >= 0) {
+          if (tq[q] >= 0) {
 #pragma unroll
-            for (int r = 0; r < 6; r++) {
+            for (int e = 0; e < 6; e++) {
               double sacc = 0.0;
 #pragma unroll
-              for (int m = 0; m < 6; m++) sacc = fma(Lb[6 * r + m], v[q][m], sacc);
-              R[36 * (size_t)tp[q] + 6 * r + c] = a[q][r] - sacc;
+              for (int m = 0; m < 6; m++) sacc = fma(Lb[6 * e + m], v[q][m], sacc);
+              R[36 * (size_t)tq[q] + 6 * e + c] = a[q][e] - sacc;
             }
           }
       }
       __syncwarp();
+      kp = kpn;
+      ext = extn;
+#pragma unroll
+      for (int q = 0; q < kFacPass; q++) tp[q] = target(jn[q], kpn);
     }
     if (!live) break;
     double* Dii = R + 36 * (size_t)di;
-    for (int t = lane; t < 36; t += 32) sM[t] = Dii[t];
-    __syncwarp();
-    inv6_warp(sM, sI, lane, ctl, d.off + i);
-    for (int t = lane; t < 36; t += 32) {
-      const double v = sI[t];
-      if (!isfinite(v)) {
-        atomicOr(&ctl->status, ST_ZERO_PIVOT);
-        atomicCAS(&ctl->pivot, 0, d.off + i + 1);
-      }
-      Dii[t] = v;
+    const int j12 = lane % 12;
+    double m[6];
+#pragma unroll
+    for (int e = 0; e < 6; e++) m[e] = j12 < 6 ? Dii[6 * e + j12] : (e == j12 - 6 ? 1.0 : 0.0);
+    bool ok = inv6_cols(m);
+#pragma unroll
+    for (int e = 0; e < 6; e++) ok = ok && isfinite(m[e]);
+    if (!ok && lane < 12) {
+      atomicOr(&ctl->status, ST_ZERO_PIVOT);
+      atomicCAS(&ctl->pivot, 0, d.off + i + 1);
     }
     __syncwarp();
-    if (vstaged) {
-      double* dst = LU + 36 * (size_t)r0;
-      for (int t = lane; t < 36 * len; t += 32) dst[t] = sR[t];
-    }
-    if (mapped)
-      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = -1;
-    // publish: every lane's stores of the row reach device scope before the
-    // flag (release) says the row is final
-    __threadfence();
+    if (lane >= 6 && lane < 12)
+#pragma unroll
+      for (int e = 0; e < 6; e++) Dii[6 * e + lane - 6] = m[e];
+    __syncwarp();
+    // the upper part, then its flag: the lane's release covers the other
+    // lanes' stores, which the warp barrier orders before it
+    const int nl = 18 * (di - r0);
+    double2* dst = reinterpret_cast<double2*>(LU + 36 * (size_t)r0);
+    const double2* src = reinterpret_cast<const double2*>(sR);
+    if (vstaged)
+      for (int t = nl + lane; t < 18 * len; t += 32) dst[t] = src[t];
     __syncwarp();
     if (lane == 0 && !(skip_first && idx == 0)) st_release_gpu(done + i, epoch);
+    if (vstaged)
+      for (int t = lane; t < nl; t += 32) dst[t] = src[t];
+    if (mapped)
+      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = -1;
+    __syncwarp();
     idx = __shfl_sync(0xffffffffu, nidx, 0);
   }
 }
