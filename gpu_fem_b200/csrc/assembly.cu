@@ -190,10 +190,25 @@ __device__ __forceinline__ void element_stiffness(ElemData& d, const Material& m
   ColumnAt c[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) c[k] = column_at(d, 8 * k + i, q);
-  double E[3], S[3];
-  // drill, then transverse shear, then (E2, E5), then (E0, E1, E3, E4)
+  // Smallest terms first, the membrane's last: fewer roundings at the size of
+  // the sum.
+  double E0[3], E1[3], E2[3], E[3], S[3];
 #pragma unroll
-  for (int k = 0; k < 3; k++) E[k] = c[k].e8, S[k] = D.r * E[k];
+  for (int k = 0; k < 3; k++) {
+    E0[k] = tying_row(d, q, 0, c[k].g);
+    E1[k] = tying_row(d, q, 1, c[k].g);
+    E2[k] = tying_row(d, q, 2, c[k].g);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    E[k] = c[k].e3, S[k] = D.b0 * E0[k] + D.b1 * E1[k] + D.d0 * c[k].e3 + D.d1 * c[k].e4;
+  mma_step(acc, E, S);
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    E[k] = c[k].e4, S[k] = D.b1 * E0[k] + D.b0 * E1[k] + D.d1 * c[k].e3 + D.d0 * c[k].e4;
+  mma_step(acc, E, S);
+#pragma unroll
+  for (int k = 0; k < 3; k++) E[k] = c[k].e5, S[k] = D.b5 * E2[k] + D.d5 * E[k];
   mma_step(acc, E, S);
 #pragma unroll
   for (int z = 3; z < 5; z++) {
@@ -201,43 +216,20 @@ __device__ __forceinline__ void element_stiffness(ElemData& d, const Material& m
     for (int k = 0; k < 3; k++) E[k] = tying_row(d, q, z, c[k].g), S[k] = D.s * E[k];
     mma_step(acc, E, S);
   }
-  {
-    double E2[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) E2[k] = tying_row(d, q, 2, c[k].g);
+  for (int k = 0; k < 3; k++) E[k] = c[k].e8, S[k] = D.r * E[k];
+  mma_step(acc, E, S);
 #pragma unroll
-    for (int k = 0; k < 3; k++) S[k] = D.a5 * E2[k] + D.b5 * c[k].e5;
-    mma_step(acc, E2, S);
+  for (int k = 0; k < 3; k++) S[k] = D.a5 * E2[k] + D.b5 * c[k].e5;
+  mma_step(acc, E2, S);
 #pragma unroll
-    for (int k = 0; k < 3; k++) E[k] = c[k].e5, S[k] = D.b5 * E2[k] + D.d5 * E[k];
-    mma_step(acc, E, S);
-  }
-  {
-    double E0[3], E1[3], E3[3], E4[3];
+  for (int k = 0; k < 3; k++)
+    S[k] = D.a0 * E0[k] + D.a1 * E1[k] + D.b0 * c[k].e3 + D.b1 * c[k].e4;
+  mma_step(acc, E0, S);
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      E0[k] = tying_row(d, q, 0, c[k].g);
-      E1[k] = tying_row(d, q, 1, c[k].g);
-      E3[k] = c[k].e3;
-      E4[k] = c[k].e4;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      S[k] = D.a0 * E0[k] + D.a1 * E1[k] + D.b0 * E3[k] + D.b1 * E4[k];
-    mma_step(acc, E0, S);
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      S[k] = D.a1 * E0[k] + D.a0 * E1[k] + D.b1 * E3[k] + D.b0 * E4[k];
-    mma_step(acc, E1, S);
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      S[k] = D.b0 * E0[k] + D.b1 * E1[k] + D.d0 * E3[k] + D.d1 * E4[k];
-    mma_step(acc, E3, S);
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      S[k] = D.b1 * E0[k] + D.b0 * E1[k] + D.d1 * E3[k] + D.d0 * E4[k];
-    mma_step(acc, E4, S);
-  }
+  for (int k = 0; k < 3; k++)
+    S[k] = D.a1 * E0[k] + D.a0 * E1[k] + D.b1 * c[k].e3 + D.b0 * c[k].e4;
+  mma_step(acc, E1, S);
   __syncwarp();  // the tables have been read
   double* K = reinterpret_cast<double*>(&d);
   int tile = 0;

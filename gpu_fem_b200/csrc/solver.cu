@@ -217,6 +217,8 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
     double f[6];
 #pragma unroll
     for (int r = 0; r < 6; r++) f[r] = __shfl_sync(0xffffffffu, m[r], c);
+    // the reciprocal of the usual pivot, while the search runs
+    double inv = 1.0 / f[c];
     int p = c;
     double best = fabs(f[c]);
 #pragma unroll
@@ -228,17 +230,20 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
       }
     }
     ok = ok && best > 0.0 && isfinite(best);
+    if (p != c) {  // the same for every lane, and rare
 #pragma unroll
-    for (int r = c + 1; r < 6; r++)
-      if (p == r) {
-        double t = m[c];
-        m[c] = m[r];
-        m[r] = t;
-        t = f[c];
-        f[c] = f[r];
-        f[r] = t;
-      }
-    m[c] *= 1.0 / f[c];
+      for (int r = c + 1; r < 6; r++)
+        if (p == r) {
+          double t = m[c];
+          m[c] = m[r];
+          m[r] = t;
+          t = f[c];
+          f[c] = f[r];
+          f[r] = t;
+        }
+      inv = 1.0 / f[c];
+    }
+    m[c] *= inv;
 #pragma unroll
     for (int r = 0; r < 6; r++)
       if (r != c) m[r] = fma(-f[r], m[c], m[r]);
@@ -252,8 +257,15 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
 // of shared memory (rows up to kFacVals blocks; longer rows are updated in
 // global memory), so the read-modify-writes of the sequential steps cost a
 // shared-memory latency. Within a row the steps k (its lower blocks) are
-// sequential; a step's updates A_ij -= L_ik U_kj over j in U(k) are spread
-// over the lanes (lane = block slot b < 5, column c < 6).
+// sequential; a step is L_ik = A_ik U_kk^{-1} and the updates A_ij -= L_ik U_kj
+// over the blocks j of U(k) that the row has, on the FP64 tensor instruction
+// m8n8k4: the 6x6 blocks are padded to 8 rows and 8 inner columns, four
+// blocks fill three tiles of 8 columns, L_ik goes from one product to the
+// next through shuffles and U(k) from L2 straight into the operands, all of
+// its first 32 blocks in flight together. (As scalar multiply-adds a step
+// took 920 instructions, which bounds batches, where every SM has rows to
+// factor all the time. Eight warps with all registers beat twelve or sixteen
+// whose loads come in two rounds or spill: an acquire drops the SM's L1.)
 //
 // Scheduling is dataflow, not level-synchronous: the warps of the CTAs a
 // problem is given take its rows in factorization order (ascending lower
@@ -273,18 +285,23 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
 // and are looked up a step ahead, before the wait; the wait polls one
 // acquiring load (the limit is checked every 64th time); the inverse stays in
 // registers; and the flag follows the upper part of the row at once (nobody
-// reads the lower part in this launch), released by one lane.
-constexpr int kFacWarps = 8;
-constexpr int kFacRow = 256;    // row blocks whose columns are staged in shared memory
-constexpr int kFacVals = 80;    // row blocks whose values are staged in shared memory
-constexpr int kFacSteps = 128;  // steps whose extent of U(k) is staged
-constexpr int kFacPass = 6;     // passes of 5 U(k) blocks loaded at the start of a step
-constexpr int kFacBatch = 2;    // passes of 5 blocks in flight per lane beyond those
-constexpr int kFacMap = 1024;   // column span of a row whose column -> slot map is kept
-// per warp: values, L_ik, U(k) extents, columns, map and the row's step order
-constexpr size_t kFacWarpSmem = sizeof(double) * (36 * kFacVals + 36) + sizeof(int2) * kFacSteps +
-                                sizeof(int32_t) * kFacRow + sizeof(int16_t) * (kFacMap + kFacRow);
-constexpr size_t kFacSmem = kFacWarps * kFacWarpSmem;
+// reads the lower part in this launch), released by one lane. Clocks of that
+// chain on a 256x128 plate, ILU(6): operands 1,150, updates 1,300, inverse
+// 2,300, stores 640, release 970, the rest is the flag's way to the waiting
+// warp. Alone, before -> now (B200): 256x128, ILU(6) 11.7 -> 6.4 ms; 61x37,
+// ILU(8) 3.9 -> 2.0 ms; the 64-plate batch 38 -> 32 ms.
+constexpr int kFacWarps = 8;      // warps a CTA counts for when CTAs are shared out
+constexpr int kFacWarpsMax = 8;  // warps of a CTA at most (its shared memory decides)
+constexpr int kFacVals = 80;      // row blocks whose values are staged at most
+constexpr int kFacSteps = 64;     // steps of a row that are staged
+constexpr int kFacMap = 1024;     // column span of a row whose column -> slot map is kept
+constexpr size_t kFacSmemMax = 226 * 1024;
+// per warp: values of `vals` blocks and one more that padding reads, the
+// steps, two lists of updates and the column map
+__host__ __device__ inline size_t fac_warp_smem(int vals) {
+  return sizeof(double) * 36 * ((size_t)vals + 1) + sizeof(int4) * kFacSteps + sizeof(int2) * 64 +
+         kFacMap;
+}
 
 __device__ __forceinline__ int find_col(const int32_t* c, int lo, int hi, int j) {
   const int end = hi;
@@ -331,26 +348,198 @@ __device__ __forceinline__ bool wait_flag(const int* flag, int want, unsigned lo
   }
 }
 
+// c += A B, lane = 4 row + k of A (8x4), 4 column + k of B (4x8), 4 row +
+// column / 2 of c (8x8): exact FP64 multiply-adds
+__device__ __forceinline__ void mma_f64(double2& c, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c.x), "+d"(c.y)
+      : "d"(a), "d"(b));
+}
+
+// A row's block values (STAGED: in the warp's shared memory, else in the
+// factor itself).
+template <bool STAGED>
+struct RowValues {
+  unsigned char* base;
+  __device__ __forceinline__ double* at(int slot) const {
+    return reinterpret_cast<double*>(base + 288u * (unsigned)slot);
+  }
+};
+
+// The lower steps of one row (r0 its first block, nlow steps). False when a
+// wait ran out.
+template <bool STAGED>
+__device__ __forceinline__ bool factor_row(const RowValues<STAGED> R, const int4* __restrict__ steps,
+                                           int nlow, int len, const int4* sS, int2* sT,
+                                           const uint8_t* sMap, int cbase, int span, bool mapped,
+                                           const int32_t* __restrict__ cols,
+                                           const int32_t* __restrict__ rcols, const double* LU,
+                                           const int* done, int epoch, unsigned long long wlim,
+                                           SweepCtl* ctl, int lane) {
+  const int row = lane >> 2, q = lane & 3;  // tile row (column of B) and inner index
+  // column 8 t + row of four blocks side by side is column co[t] of block
+  // bo[t]; columns 8 t + 2 q and the next one belong to block bc[t]
+  int bo[3], bc[3], cc[3];
+  const double* LUt[3];
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    bo[t] = (8 * t + row) / 6;
+    LUt[t] = LU + 6 * q + (8 * t + row) % 6;
+    bc[t] = (8 * t + 2 * q) / 6;
+    cc[t] = 6 * row + (8 * t + 2 * q) % 6;
+  }
+  const bool inner = q < 2, rows6 = row < 6;  // lanes with a second inner index / a block row
+  // step t: {slot, k, first and end block of U(k)}
+  auto step = [&](int t) { return t < kFacSteps ? sS[t] : __ldg(steps + t); };
+  // Lists the updates of 32 blocks of U(k) from block jp0 on (the lane's
+  // block has column j, -1: none), padded to a multiple of four; their number.
+  auto list_updates = [&](int2* list, int j, int jp0, int slot_k) {
+    int slot = -1;
+    if (j >= 0) {
+      if (mapped) {
+        const int o = j - cbase;
+        const int m = o < span ? sMap[o] : 255;
+        slot = m < 255 ? m : -1;
+      } else {
+        slot = find_col(rcols, slot_k + 1, len, j);
+      }
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, slot >= 0);
+    const int n = __popc(hit);
+    if (slot >= 0) list[__popc(hit & ((1u << lane) - 1u))] = make_int2(9 * (jp0 + lane), slot);
+    if (lane < ((4 - n) & 3)) list[n + lane] = make_int2(9 * (jp0 - 1), STAGED ? len : 0);
+    return n;
+  };
+  double b0[24], b1[24];  // U(k) operands of eight groups of four blocks
+#pragma unroll
+  for (int t = 0; t < 24; t++) b0[t] = b1[t] = 0.0;
+  auto load_groups = [&](const int2* list, int n) {
+#pragma unroll
+    for (int g = 0; g < 8; g++)
+      if (4 * g < n)
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+          const double* src = LUt[t] + 4 * (size_t)(unsigned)list[4 * g + bo[t]].x;
+          b0[3 * g + t] = __ldcg(src);
+          if (inner) b1[3 * g + t] = __ldcg(src + 24);
+        }
+  };
+  auto update_groups = [&](const int2* list, int n, double l0, double l1) {
+#pragma unroll
+    for (int h = 0; h < 8; h += 2) {  // two groups at a time
+      if (4 * h >= n) break;
+      const bool two = 4 * (h + 1) < n;
+      // the products of a block are summed by themselves and subtracted once:
+      // one rounding a step at the size of A_ij
+      double2 c[6], s[6];
+      unsigned at[6];
+#pragma unroll
+      for (int t = 0; t < 6; t++) {
+        c[t] = s[t] = make_double2(0.0, 0.0);
+        if (t < 3 || two) {
+          at[t] = 288u * (unsigned)list[4 * (h + t / 3) + bc[t % 3]].y + 8u * (unsigned)cc[t % 3];
+          if (rows6) c[t] = *reinterpret_cast<double2*>(R.base + at[t]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+        if (t < 3 || two) mma_f64(s[t], l0, b0[3 * h + t]);
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+        if (t < 3 || two) mma_f64(s[t], l1, b1[3 * h + t]);
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+        if ((t < 3 || two) && rows6 && 4 * (h + t / 3) + bc[t % 3] < n)
+          *reinterpret_cast<double2*>(R.base + at[t]) =
+              make_double2(c[t].x - s[t].x, c[t].y - s[t].y);
+    }
+  };
+  // this step and the updates of its first 32 blocks
+  int nt = 0, cur = 0;
+  int4 s0 = make_int4(0, 0, 0, 0);
+  if (nlow > 0) {
+    s0 = step(0);
+    nt = list_updates(sT, s0.z + lane < s0.w ? __ldg(cols + s0.z + lane) : -1, s0.z, s0.x);
+  }
+  __syncwarp();
+  unsigned ready = 0;  // bit z: the row of step (window start + z) is final
+  for (int st = 0; st < nlow; st++) {
+    if ((st & 31) == 0) {
+      // the flags of the next 32 steps, one per lane; a lane that sees its
+      // row final acquires it for the warp (the warp barrier below orders
+      // that acquire before every lane's later loads)
+      const int f = st + lane < nlow ? (ld_acquire_gpu(done + step(st + lane).y) == epoch) : 1;
+      ready = __ballot_sync(0xffffffffu, f);
+      __syncwarp();
+    }
+    // the next step's columns, in flight during this one
+    int jn = -1;
+    int4 s1 = s0;
+    if (st + 1 < nlow) {
+      s1 = step(st + 1);
+      if (s1.z + lane < s1.w) jn = __ldg(cols + s1.z + lane);
+    }
+    double* Aik = R.at(s0.x);
+    const double a0 = rows6 ? Aik[6 * row + q] : 0.0;
+    const double a1 = rows6 && inner ? Aik[6 * row + 4 + q] : 0.0;
+    if (!((ready >> (st & 31)) & 1u)) {
+      int ok = lane == 0 ? (int)wait_flag(done + s0.y, epoch, wlim, ctl) : 0;
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      __syncwarp();
+      if (!ok) return false;
+    }
+    // U_kk^{-1} and up to 32 blocks of U(k), all in flight
+    const double* Ukk = LU + 36 * (size_t)(s0.z - 1) + 6 * q + row;
+    const double k0 = rows6 ? __ldcg(Ukk) : 0.0;
+    const double k1 = rows6 && inner ? __ldcg(Ukk + 24) : 0.0;
+    const int2* list = sT + 32 * cur;
+    load_groups(list, nt);
+    double2 l = make_double2(0.0, 0.0);
+    mma_f64(l, a0, k0);
+    mma_f64(l, a1, k1);
+    if (rows6 && q < 3) *reinterpret_cast<double2*>(Aik + 6 * row + 2 * q) = l;
+    // column q (and 4 + q) of L_ik for the updates
+    const int quad = lane & ~3;
+    const double x0 = __shfl_sync(0xffffffffu, l.x, quad + (q >> 1));
+    const double y0 = __shfl_sync(0xffffffffu, l.y, quad + (q >> 1));
+    const double x1 = __shfl_sync(0xffffffffu, l.x, quad + 2);
+    const double y1 = __shfl_sync(0xffffffffu, l.y, quad + 2);
+    const double l0 = (q & 1) ? y0 : x0, l1 = !inner ? 0.0 : (q & 1) ? y1 : x1;
+    update_groups(list, nt, l0, l1);
+    // the rest of U(k), beyond its first 32 blocks
+    for (int jb = s0.z + 32; jb < s0.w; jb += 32) {
+      __syncwarp();
+      const int n = list_updates(sT + 32 * cur, jb + lane < s0.w ? __ldg(cols + jb + lane) : -1, jb, s0.x);
+      __syncwarp();
+      load_groups(list, n);
+      update_groups(list, n, l0, l1);
+    }
+    cur ^= 1;
+    nt = list_updates(sT + 32 * cur, jn, s1.z, s1.x);
+    s0 = s1;
+    __syncwarp();
+  }
+  return true;
+}
+
 // cta_prob[blockIdx.x]: the problem a CTA works on; grab[p]: problem p's row
-// counter (zero at launch).
-__global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __restrict__ P,
-                                                            const int32_t* __restrict__ cta_prob,
-                                                            int* __restrict__ grab, int epoch,
-                                                            SweepCtl* ctl) {
+// counter (zero at launch). vals: blocks of a row that are staged.
+__global__ void __launch_bounds__(kFacWarpsMax * 32) bfactor_df(const ProbDev* __restrict__ P,
+                                                               const int32_t* __restrict__ cta_prob,
+                                                               int* __restrict__ grab, int epoch,
+                                                               int vals, SweepCtl* ctl) {
   extern __shared__ __align__(16) unsigned char fsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* ws = fsm + (size_t)warp * kFacWarpSmem;
-  double* sR = reinterpret_cast<double*>(ws);  // staged row values
-  double* Lb = sR + 36 * kFacVals;             // L_ik of the current step
-  int2* sU = reinterpret_cast<int2*>(Lb + 36);  // step t -> blocks of U(k)
-  int32_t* sC = reinterpret_cast<int32_t*>(sU + kFacSteps);
-  int16_t* sMap = reinterpret_cast<int16_t*>(sC + kFacRow);  // column - base -> slot - r0, or -1
-  int16_t* sOrd = sMap + kFacMap;                              // step t -> slot - r0
-  for (int t = lane; t < kFacMap; t += 32) sMap[t] = -1;
+  unsigned char* ws = fsm + (unsigned)warp * (unsigned)fac_warp_smem(vals);
+  double2* sR = reinterpret_cast<double2*>(ws);  // staged row values
+  int4* sS = reinterpret_cast<int4*>(ws + 288 * (vals + 1));
+  int2* sT = reinterpret_cast<int2*>(sS + kFacSteps);  // updates of this and the next step
+  uint8_t* sMap = reinterpret_cast<uint8_t*>(sT + 64);  // column - base -> slot, or 255
+  for (int t = lane; t < kFacMap; t += 32) sMap[t] = 255;
+  if (lane < 18) sR[18 * vals + lane] = make_double2(0.0, 0.0);
   __syncwarp();
-  const int b = lane / 6, c = lane % 6;  // update slot and column (lanes 30, 31 idle)
   const int prob = cta_prob[blockIdx.x];
-  const ProbDev d = P[prob];
+  const ProbDev& d = P[prob];
   int* counter = grab + prob;
   int* done = d.done;
   const unsigned long long wlim = g_wait_ns;
@@ -358,209 +547,53 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
   const int32_t* rowp = d.prowp;
   const int32_t* cols = d.pcols;
   const int32_t* diag = d.pdiag;
+  const int4* steps = d.psteps;
+  const int32_t* rows = d.levLrows;
+  const int n = d.n, off = d.off;
   double* LU = d.LU64;
   int idx = lane == 0 ? atomicAdd(counter, 1) : 0;
   idx = __shfl_sync(0xffffffffu, idx, 0);
-  bool live = true;
-  while (idx < d.n && live) {
-    const int nidx = lane == 0 ? atomicAdd(counter, 1) : 0;  // the next row, in flight meanwhile
-    const int i = d.levLrows[idx];
-    const int r0 = rowp[i], r1 = rowp[i + 1], di = diag[i], len = r1 - r0;
-    const bool cstaged = len <= kFacRow;
-    const bool vstaged = len <= kFacVals;
-    const int32_t* rc = cstaged ? sC - r0 : cols;  // rc[kp] = column of slot kp
-    double* R = vstaged ? sR - 36 * (size_t)r0 : LU;  // R[36 kp + e] = entry e of slot kp
-    // extent of U(k) for the steps, staged ahead (columns read from global)
-    for (int t = lane; t < min(di - r0, kFacSteps); t += 32) {
-      const int k = cols[d.pord[r0 + t]];
-      sU[t] = make_int2(diag[k] + 1, rowp[k + 1]);
-    }
-    if (cstaged) {
-      for (int t = lane; t < len; t += 32) sC[t] = cols[r0 + t];
-      for (int t = lane; t < di - r0; t += 32) sOrd[t] = (int16_t)(d.pord[r0 + t] - r0);
-    }
-    // slot of the row's step t (r0 <= t < di)
-    auto step_slot = [&](int t) { return cstaged ? r0 + sOrd[t - r0] : d.pord[t]; };
+  int i = idx < n ? rows[idx] : 0;
+  int r0 = rowp[i], r1 = rowp[i + 1], di = diag[i];
+  while (idx < n) {
+    int nidx = lane == 0 ? atomicAdd(counter, 1) : 0;  // the next row, in flight meanwhile
+    const int len = r1 - r0, nlow = di - r0;
+    const bool vstaged = len <= vals;
+    for (int t = lane; t < min(nlow, kFacSteps); t += 32) sS[t] = __ldg(steps + r0 + t);
     // column -> slot map of the row when its column span fits (binary
     // searches otherwise)
     const int cbase = cols[r0], span = cols[r1 - 1] - cbase + 1;
-    const bool mapped = span <= kFacMap;
+    const bool mapped = span <= kFacMap && len < 255;
     if (mapped)
-      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = (int16_t)t;
+      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = (uint8_t)t;
+    double2* dst = reinterpret_cast<double2*>(LU + 36 * (size_t)r0);
     if (vstaged) {
-      // four 16-byte loads in flight per lane
-      const double2* src = reinterpret_cast<const double2*>(LU + 36 * (size_t)r0);
-      double2* dst = reinterpret_cast<double2*>(sR);
+      // eight 16-byte loads in flight per lane
       const int nv = 18 * len;
-      for (int t0 = 0; t0 < nv; t0 += 128) {
-        double2 v[4];
+      for (int t0 = lane; t0 < nv; t0 += 256) {
+        double2 v[8];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int t = t0 + 32 * q + lane;
-          v[q] = t < nv ? src[t] : make_double2(0.0, 0.0);
-        }
+        for (int z = 0; z < 8; z++)
+          if (t0 + 32 * z < nv) v[z] = __ldcg(dst + t0 + 32 * z);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int t = t0 + 32 * q + lane;
-          if (t < nv) dst[t] = v[q];
-        }
+        for (int z = 0; z < 8; z++)
+          if (t0 + 32 * z < nv) sR[t0 + 32 * z] = v[z];
       }
     }
     __syncwarp();
-    auto extent = [&](int st, int kp) {
-      if (st - r0 < kFacSteps) return sU[st - r0];
-      const int k = rc[kp];
-      return make_int2(diag[k] + 1, rowp[k + 1]);
-    };
-    // slot of the row that column j of U(k) updates, or -1 (j < 0: none)
-    auto target = [&](int j, int kp) {
-      if (j < 0) return -1;
-      if (!mapped) return find_col(rc, kp + 1, r1, j);
-      const int off = j - cbase;
-      const int m = off < span ? sMap[off] : -1;
-      return m >= 0 ? r0 + m : -1;
-    };
-    // this step's slot, extent of U(k) and targets of its first blocks
-    int kp = r0, tp[kFacPass];
-    int2 ext = make_int2(0, 0);
-    if (r0 < di) {
-      kp = step_slot(r0);
-      ext = extent(r0, kp);
-#pragma unroll
-      for (int q = 0; q < kFacPass; q++) {
-        const int jp = ext.x + 5 * q + b;
-        tp[q] = target(lane < 30 && jp < ext.y ? cols[jp] : -1, kp);
-      }
-    }
-    unsigned ready = 0;  // bit s: the row of step (window start + s) is final
-    for (int st = r0; st < di; st++) {
-      const int s = (st - r0) & 31;
-      if (s == 0) {
-        // the flags of the next 32 steps, one per lane; a lane that sees
-        // its row final acquires it for the warp (the warp barrier below
-        // orders that acquire before every lane's later loads)
-        const int q = st + lane;
-        const int f = q < di ? (ld_acquire_gpu(done + rc[step_slot(q)]) == epoch) : 1;
-        ready = __ballot_sync(0xffffffffu, f);
-        __syncwarp();
-      }
-      const int k = rc[kp], u0 = ext.x, u1 = ext.y;
-      // the next step's columns, in flight during this one
-      int kpn = kp, jn[kFacPass];
-      int2 extn = make_int2(0, 0);
-      if (st + 1 < di) {
-        kpn = step_slot(st + 1);
-        extn = extent(st + 1, kpn);
-      }
-#pragma unroll
-      for (int q = 0; q < kFacPass; q++) {
-        const int jp = extn.x + 5 * q + b;
-        jn[q] = lane < 30 && jp < extn.y ? __ldg(cols + jp) : -1;
-      }
-      if (!((ready >> s) & 1u)) {
-        int ok = lane == 0 ? (int)wait_flag(done + k, epoch, wlim, ctl) : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        __syncwarp();
-        if (!ok) {
-          live = false;
-          break;
-        }
-      }
-      // U_kk^{-1} and the first kFacPass x 5 blocks of U(k), all in flight
-      const double* Ukk = LU + 36 * (size_t)(u0 - 1);
-      const int r = lane / 6, cc = lane % 6, r2 = (lane + 32) / 6, c2 = (lane + 32) % 6;
-      double uk[6], uk2[6], u[kFacPass][6];
-#pragma unroll
-      for (int m = 0; m < 6; m++) uk[m] = __ldcg(Ukk + 6 * m + cc);
-#pragma unroll
-      for (int m = 0; m < 6; m++) uk2[m] = lane < 4 ? __ldcg(Ukk + 6 * m + c2) : 0.0;
-#pragma unroll
-      for (int q = 0; q < kFacPass; q++) {
-        const double* src = LU + 36 * (size_t)(u0 + 5 * q + b) + c;
-#pragma unroll
-        for (int m = 0; m < 6; m++) u[q][m] = tp[q] >= 0 ? __ldcg(src + 6 * m) : 0.0;
-      }
-      double* Aik = R + 36 * (size_t)kp;
-      double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-      for (int m = 0; m < 6; m++) s0 = fma(Aik[6 * r + m], uk[m], s0);
-      if (lane < 4)
-#pragma unroll
-        for (int m = 0; m < 6; m++) s1 = fma(Aik[6 * r2 + m], uk2[m], s1);
-      __syncwarp();
-      Lb[lane] = s0;
-      Aik[lane] = s0;
-      if (lane < 4) {
-        Lb[32 + lane] = s1;
-        Aik[32 + lane] = s1;
-      }
-      __syncwarp();
-      {
-        // the targets are distinct slots of this row: all their reads before
-        // any write
-        double lb[36];  // L_ik in registers for the updates
-#pragma unroll
-        for (int t = 0; t < 36; t += 2) {
-          const double2 v = *reinterpret_cast<const double2*>(Lb + t);
-          lb[t] = v.x, lb[t + 1] = v.y;
-        }
-        double a[kFacPass][6];
-#pragma unroll
-        for (int q = 0; q < kFacPass; q++)
-#pragma unroll
-          for (int e = 0; e < 6; e++) a[q][e] = tp[q] >= 0 ? R[36 * (size_t)tp[q] + 6 * e + c] : 0.0;
-#pragma unroll
-        for (int q = 0; q < kFacPass; q++)
-          if (tp[q] >= 0) {
-#pragma unroll
-            for (int e = 0; e < 6; e++) {
-              double sacc = 0.0;
-#pragma unroll
-              for (int m = 0; m < 6; m++) sacc = fma(lb[6 * e + m], u[q][m], sacc);
-              R[36 * (size_t)tp[q] + 6 * e + c] = a[q][e] - sacc;
-            }
-          }
-      }
-      // the rest of U(k) (rows longer than the prefetch), kFacBatch passes at a time
-      for (int jb = u0 + 5 * kFacPass; jb < u1; jb += 5 * kFacBatch) {
-        int jt[kFacBatch];
-        double v[kFacBatch][6];
-#pragma unroll
-        for (int q = 0; q < kFacBatch; q++) {
-          const int jp = jb + 5 * q + b;
-          const bool in = lane < 30 && jp < u1;
-          jt[q] = in ? __ldg(cols + jp) : -1;
-#pragma unroll
-          for (int m = 0; m < 6; m++) v[q][m] = in ? __ldcg(LU + 36 * (size_t)jp + 6 * m + c) : 0.0;
-        }
-        int tq[kFacBatch];
-#pragma unroll
-        for (int q = 0; q < kFacBatch; q++) tq[q] = target(jt[q], kp);
-        double a[kFacBatch][6];
-#pragma unroll
-        for (int q = 0; q < kFacBatch; q++)
-#pragma unroll
-          for (int e = 0; e < 6; e++) a[q][e] = tq[q] >= 0 ? R[36 * (size_t)tq[q] + 6 * e + c] : 0.0;
-#pragma unroll
-        for (int q = 0; q < kFacBatch; q++)
-          if (tq[q] >= 0) {
-#pragma unroll
-            for (int e = 0; e < 6; e++) {
-              double sacc = 0.0;
-#pragma unroll
-              for (int m = 0; m < 6; m++) sacc = fma(Lb[6 * e + m], v[q][m], sacc);
-              R[36 * (size_t)tq[q] + 6 * e + c] = a[q][e] - sacc;
-            }
-          }
-      }
-      __syncwarp();
-      kp = kpn;
-      ext = extn;
-#pragma unroll
-      for (int q = 0; q < kFacPass; q++) tp[q] = target(jn[q], kpn);
-    }
+    bool live;
+    if (vstaged)
+      live = factor_row<true>(RowValues<true>{ws}, steps + r0, nlow, len, sS, sT, sMap,
+                              cbase, span, mapped, cols, cols + r0, LU, done, epoch, wlim, ctl, lane);
+    else
+      live = factor_row<false>(RowValues<false>{reinterpret_cast<unsigned char*>(LU + 36 * (size_t)r0)}, steps + r0, nlow,
+                               len, sS, sT, sMap, cbase, span, mapped, cols, cols + r0, LU, done,
+                               epoch, wlim, ctl, lane);
     if (!live) break;
-    double* Dii = R + 36 * (size_t)di;
+    // the next row's extent, in flight during the end of this one
+    nidx = __shfl_sync(0xffffffffu, nidx, 0);
+    const int ni = nidx < n ? rows[nidx] : 0;
+    double* Dii = vstaged ? reinterpret_cast<double*>(ws + 288 * nlow) : LU + 36 * (size_t)di;
     const int j12 = lane % 12;
     double m[6];
 #pragma unroll
@@ -570,7 +603,7 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
     for (int e = 0; e < 6; e++) ok = ok && isfinite(m[e]);
     if (!ok && lane < 12) {
       atomicOr(&ctl->status, ST_ZERO_PIVOT);
-      atomicCAS(&ctl->pivot, 0, d.off + i + 1);
+      atomicCAS(&ctl->pivot, 0, off + i + 1);
     }
     __syncwarp();
     if (lane >= 6 && lane < 12)
@@ -579,19 +612,40 @@ __global__ void __launch_bounds__(kFacWarps * 32) bfactor_df(const ProbDev* __re
     __syncwarp();
     // the upper part, then its flag: the lane's release covers the other
     // lanes' stores, which the warp barrier orders before it
-    const int nl = 18 * (di - r0);
-    double2* dst = reinterpret_cast<double2*>(LU + 36 * (size_t)r0);
-    const double2* src = reinterpret_cast<const double2*>(sR);
-    if (vstaged)
-      for (int t = nl + lane; t < 18 * len; t += 32) dst[t] = src[t];
+    if (vstaged) {
+#pragma unroll 4
+      for (int t = 18 * nlow + lane; t < 18 * len; t += 32) dst[t] = sR[t];
+    }
     __syncwarp();
     if (lane == 0 && !(skip_first && idx == 0)) st_release_gpu(done + i, epoch);
-    if (vstaged)
-      for (int t = lane; t < nl; t += 32) dst[t] = src[t];
+    const int nr0 = rowp[ni], nr1 = rowp[ni + 1], ndi = diag[ni];
+    if (vstaged) {
+#pragma unroll 4
+      for (int t = lane; t < 18 * nlow; t += 32) dst[t] = sR[t];
+    }
     if (mapped)
-      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = -1;
+      for (int t = lane; t < len; t += 32) sMap[cols[r0 + t] - cbase] = 255;
     __syncwarp();
-    idx = __shfl_sync(0xffffffffu, nidx, 0);
+    idx = nidx;
+    i = ni;
+    r0 = nr0;
+    r1 = nr1;
+    di = ndi;
+  }
+}
+
+// Steps of every row for the factorization: {slot of the row, row k, first
+// block and end of U(k)} in step order.
+__global__ void step_table_kernel(int n, const int32_t* __restrict__ rowp,
+                                  const int32_t* __restrict__ cols,
+                                  const int32_t* __restrict__ diag,
+                                  const int32_t* __restrict__ ord, int4* __restrict__ steps) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= n) return;
+  const int r0 = rowp[i];
+  for (int t = r0 + lane; t < diag[i]; t += 32) {
+    const int kp = ord[t], k = cols[kp];
+    steps[t] = make_int4(kp - r0, k, diag[k] + 1, rowp[k + 1]);
   }
 }
 
@@ -1816,8 +1870,9 @@ struct gf_precond {
   DevBuf<int32_t> d_rowp, d_cols, d_diag, d_amap;
   DevBuf<int32_t> d_levLptr, d_levLrows;  // factorization order
   DevBuf<int32_t> d_done;                  // per row: epoch of the factorization that finished it
-  DevBuf<int32_t> d_ord;                   // per row: the order of its factorization steps
+  DevBuf<int4> d_steps;                    // per row: its factorization steps in order
   long long fwork = 0;                     // block updates of one factorization
+  int maxrow = 0;                          // blocks of the longest row
   int sym_gpu = 0;                         // ILU(k) pattern computed on the GPU
   double sym_ms = 0.0, setup_ms = 0.0;     // host wall time of the pattern / of the whole setup
   DevBuf<double> d_lu;
@@ -2390,7 +2445,8 @@ struct gf_batch {
   DevBuf<double> d_tmp, d_b, d_x;
   int nchunks = 0;
   DevBuf<int32_t> d_cprob, d_pstart;
-  int fac_grid = 0;                  // CTAs of the dataflow factorization
+  int fac_grid = 0;                  // CTAs of the dataflow factorization,
+  int fac_vals = 0, fac_warps = 0;   // row blocks staged per warp, warps of a CTA
   DevBuf<int32_t> d_fcta, d_fgrab;   // problem of each CTA; per-problem row counters
   DevBuf<int64_t> d_clo, d_chi;
   DevBuf<PermEntry> d_perm_b, d_perm_x, d_perm_out;
@@ -2590,7 +2646,7 @@ static gf_status upload_desc(gf_batch* B) {
     d.LU64 = p->d_lu.p;
     d.nlevL = p->nlevL;
     d.done = p->d_done.p;
-    d.pord = p->d_ord.p;
+    d.psteps = p->d_steps.p;
     d.nlevU = p->nlevU;
     d.levLptr = p->d_levLptr.p;
     d.levLrows = p->d_levLrows.p;
@@ -2654,6 +2710,11 @@ static gf_status batch_build(gf_batch* B) {
     std::vector<int32_t> cta_prob;
     fac_plan(B->pcs, ctas, cta_prob);
     B->fac_grid = (int)cta_prob.size();
+    // stage the longest row (up to kFacVals blocks); as many warps as then fit
+    int most = 8;
+    for (auto* p : B->pcs) most = std::max(most, p->maxrow);
+    B->fac_vals = std::min(most, kFacVals);
+    B->fac_warps = (int)std::min<size_t>(kFacWarpsMax, kFacSmemMax / fac_warp_smem(B->fac_vals)) & ~1;
     up(B->d_fcta.upload(cta_prob));
     up(B->d_fgrab.alloc(np));
   }
@@ -2896,9 +2957,10 @@ static gf_status batch_factor(gf_batch* B, cudaStream_t st) {
     GF_CUDA(cudaMemsetAsync(B->d_fgrab.p, 0, sizeof(int32_t) * B->np, st));
     ::gf::count_launch();
     GF_CUDA(cudaFuncSetAttribute(bfactor_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kFacSmem));
-    bfactor_df<<<(unsigned)B->fac_grid, kFacWarps * 32, kFacSmem, st>>>(
-        B->d_desc.p, B->d_fcta.p, B->d_fgrab.p, epoch, B->d_ctl.p);
+                                 (int)kFacSmemMax));
+    bfactor_df<<<(unsigned)B->fac_grid, B->fac_warps * 32,
+                 B->fac_warps * fac_warp_smem(B->fac_vals), st>>>(
+        B->d_desc.p, B->d_fcta.p, B->d_fgrab.p, epoch, B->fac_vals, B->d_ctl.p);
   }
   GF_CHECK_LAUNCH();
   for (int k = 0; k < B->np; k++) {
@@ -3295,12 +3357,22 @@ gf_status gf_precond_create_ex(gf_assembler* a, int32_t fill_level, int32_t prec
   {
     std::vector<int32_t> ord;
     step_order(p->pat, diag, p->lvL, ord);
-    up(p->d_ord.upload(ord));
+    DevBuf<int32_t> d_ord;
+    up(d_ord.upload(ord));
+    up(p->d_steps.alloc((size_t)p->pat.nnz()));
+    if (e == cudaSuccess) {
+      step_table_kernel<<<(unsigned)((n + 7) / 8), 256>>>(n, p->d_rowp.p, p->d_cols.p, p->d_diag.p,
+                                                          d_ord.p, p->d_steps.p);
+      ::gf::count_launch();
+      up(cudaGetLastError());
+      up(cudaStreamSynchronize(nullptr));  // d_ord ends here
+    }
   }
   if (e == cudaSuccess) up(cudaMemset(p->d_done.p, 0, sizeof(int32_t) * (size_t)n));
   // block updates of one factorization: per step (i, k) the block L_ik and
   // one update per block of U(k)
   p->fwork = 0;
+  for (int i = 0; i < n; i++) p->maxrow = std::max(p->maxrow, p->pat.rowp[i + 1] - p->pat.rowp[i]);
   for (int i = 0; i < n; i++)
     for (int kp = p->pat.rowp[i]; kp < diag[i]; kp++) {
       const int k = p->pat.cols[kp];
