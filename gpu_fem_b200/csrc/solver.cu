@@ -1686,7 +1686,6 @@ struct GmArrays {
   double* cs;      // np * m
   double* ss;      // np * m
   double* y;       // np * m
-  double* h;       // np * (m+1)
   double* hn;      // np
   double* target;  // np
   int* jcnt;       // np
@@ -1694,28 +1693,38 @@ struct GmArrays {
   int* live;       // np
 };
 
-// h_p[i] = sum over p's chunks; H_p[i][jj] (+)= h_p[i]
-__global__ void seg_reduce_dots(const double* partial, Chunks C, int jj, int m, GmArrays G,
-                                int acc) {
-  const int p = blockIdx.x;
-  if (!G.run[p]) return;
-  for (int i = threadIdx.x; i <= jj; i += blockDim.x) {
-    double s = 0.0;
-    for (int c = C.pstart[p]; c < C.pstart[p + 1]; c++) s += partial[(size_t)i * C.n + c];
-    G.h[(size_t)p * (m + 1) + i] = s;
-    double* Hij = &G.H[(size_t)p * (m + 1) * m + (size_t)i * m + jj];
-    *Hij = acc ? *Hij + s : s;
-  }
+// Sum of v[c] over the chunks c0 .. c1 - 1 of a problem by one warp (every
+// lane returns it; the order depends on the problem's own chunks alone).
+__device__ __forceinline__ double chunk_sum(const double* v, int c0, int c1, int lane) {
+  double s = 0.0;
+  for (int c = c0 + lane; c < c1; c += 32) s += v[c];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
 }
-// w -= sum_{i<=jj} h_p[i] V_i over chunk c; optional per-chunk |w|^2
-__global__ void seg_update(const double* __restrict__ V, double* __restrict__ w, size_t N,
-                           int jj, int m, Chunks C, GmArrays G, double* pnorm) {
+// h_p[i] = sum of the dots' partials over p's chunks, by every chunk for
+// itself (no launch of its own: a step of a small problem is a row of
+// launches); the problem's first chunk also keeps H_p[i][jj] (+)= h_p[i].
+// Then w -= sum_{i<=jj} h_p[i] V_i over chunk c; optional per-chunk |w|^2.
+__global__ void __launch_bounds__(kRedThreads)
+    seg_update(const double* __restrict__ V, double* __restrict__ w, size_t N, int jj, int m,
+               Chunks C, GmArrays G, const double* __restrict__ partial, int acc_h, double* pnorm) {
   __shared__ double sh[32];
   __shared__ double hs[1024];
   const int c = blockIdx.x;
   const int p = C.prob[c];
   if (!G.run[p]) return;
-  for (int i = threadIdx.x; i <= jj; i += blockDim.x) hs[i] = G.h[(size_t)p * (m + 1) + i];
+  const int c0 = C.pstart[p], c1 = C.pstart[p + 1], lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i <= jj; i += kRedThreads / 32) {
+    const double s = chunk_sum(partial + (size_t)i * C.n, c0, c1, lane);
+    if (lane == 0) {
+      hs[i] = s;
+      if (c == c0) {
+        double* Hij = &G.H[(size_t)p * (m + 1) * m + (size_t)i * m + jj];
+        *Hij = acc_h ? *Hij + s : s;
+      }
+    }
+  }
   __syncthreads();
   const int64_t lo = C.lo[c], hi = C.hi[c];
   double acc = 0.0;
@@ -1752,14 +1761,17 @@ __global__ void seg_norm_out(const double* pnorm, Chunks C, int np, const int* m
   for (int c = C.pstart[p]; c < C.pstart[p + 1]; c++) s += pnorm[c];
   out[p] = sqrt(s);
 }
-__global__ void seg_norm_finish(const double* pnorm, Chunks C, int np, int jj, int m,
-                                GmArrays G) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np || !G.run[p]) return;
-  double s = 0.0;
-  for (int c = C.pstart[p]; c < C.pstart[p + 1]; c++) s += pnorm[c];
-  G.hn[p] = sqrt(s);
-  G.H[(size_t)p * (m + 1) * m + (size_t)(jj + 1) * m + jj] = G.hn[p];
+// dst = src / |w|: the norm from the update's per-chunk sums, by every chunk
+// for itself
+__global__ void __launch_bounds__(kRedThreads)
+    seg_normalize(const double* __restrict__ src, double* __restrict__ dst, Chunks C,
+                  const int* __restrict__ run, const double* __restrict__ pnorm) {
+  const int c = blockIdx.x;
+  const int p = C.prob[c];
+  if (!run[p]) return;
+  const double hn = sqrt(chunk_sum(pnorm, C.pstart[p], C.pstart[p + 1], threadIdx.x & 31));
+  const double inv = hn > 0.0 ? 1.0 / hn : 0.0;
+  for (int64_t t = C.lo[c] + threadIdx.x; t < C.hi[c]; t += blockDim.x) dst[t] = src[t] * inv;
 }
 __global__ void seg_scale(const double* __restrict__ src, double* __restrict__ dst, Chunks C,
                           const int* __restrict__ run, const double* __restrict__ hn) {
@@ -1769,31 +1781,49 @@ __global__ void seg_scale(const double* __restrict__ src, double* __restrict__ d
   const double inv = hn[p] > 0.0 ? 1.0 / hn[p] : 0.0;
   for (int64_t t = C.lo[c] + threadIdx.x; t < C.hi[c]; t += blockDim.x) dst[t] = src[t] * inv;
 }
-// Givens update of column jj (examples/iterative/gmres.cu:672-699) per problem
-__global__ void bgivens(int np, int jj, int m, int step_limit, GmArrays G) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np || !G.run[p]) return;
+// Givens update of column jj (examples/iterative/gmres.cu:672-699), one warp
+// per problem. The column's running entry stays in a register, so the loads of
+// the rotations do not wait for one another. seen (host memory): the problem's
+// run flag and, behind the flags, the sweeps' status, for the host's poll.
+__global__ void bgivens(int np, int jj, int m, int step_limit, GmArrays G,
+                        const double* __restrict__ pnorm, Chunks C, const SweepCtl* ctl,
+                        volatile int* seen) {
+  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (p >= np) return;
+  if (p == 0 && lane == 0) seen[np] = ctl->status;
+  if (!G.run[p]) {
+    if (lane == 0) seen[p] = 0;
+    return;
+  }
+  const double hn = sqrt(chunk_sum(pnorm, C.pstart[p], C.pstart[p + 1], lane));
+  if (lane != 0) return;
   double* H = G.H + (size_t)p * (m + 1) * m;
   double* g = G.g + (size_t)p * (m + 1);
   double* cs = G.cs + (size_t)p * m;
   double* ss = G.ss + (size_t)p * m;
+  double a = H[jj];
+#pragma unroll 4
   for (int i = 0; i < jj; i++) {
-    const double a = H[(size_t)i * m + jj], c = H[(size_t)(i + 1) * m + jj];
-    H[(size_t)i * m + jj] = cs[i] * a + ss[i] * c;
-    H[(size_t)(i + 1) * m + jj] = -ss[i] * a + cs[i] * c;
+    const double c = H[(size_t)(i + 1) * m + jj], ci = cs[i], si = ss[i];
+    H[(size_t)i * m + jj] = ci * a + si * c;
+    a = -si * a + ci * c;
   }
-  const double a = H[(size_t)jj * m + jj], c = H[(size_t)(jj + 1) * m + jj];
+  const double c = hn;
   const double hyp = sqrt(a * a + c * c);
-  cs[jj] = hyp > 0.0 ? a / hyp : 1.0;
-  ss[jj] = hyp > 0.0 ? c / hyp : 0.0;
-  H[(size_t)jj * m + jj] = cs[jj] * a + ss[jj] * c;
+  const double cj = hyp > 0.0 ? a / hyp : 1.0, sj = hyp > 0.0 ? c / hyp : 0.0;
+  cs[jj] = cj;
+  ss[jj] = sj;
+  H[(size_t)jj * m + jj] = cj * a + sj * c;
   H[(size_t)(jj + 1) * m + jj] = 0.0;
-  g[jj + 1] = -ss[jj] * g[jj];
-  g[jj] = cs[jj] * g[jj];
+  const double gj = g[jj], gn = -sj * gj;
+  g[jj + 1] = gn;
+  g[jj] = cj * gj;
+  G.hn[p] = hn;
   G.jcnt[p] = jj + 1;
-  if (fabs(g[jj + 1]) <= G.target[p] || G.hn[p] == 0.0 || !isfinite(g[jj + 1]) ||
-      jj + 1 >= step_limit)
-    G.run[p] = 0;
+  const int run =
+      !(fabs(gn) <= G.target[p] || hn == 0.0 || !isfinite(gn) || jj + 1 >= step_limit);
+  G.run[p] = run;
+  seen[p] = run;
 }
 __global__ void bbacksolve(int np, int m, GmArrays G) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2446,6 +2476,84 @@ static size_t sweep_smem(const gf_precond* p, int which) {
 }
 }  // namespace gf
 
+// Host memory and events through which a solve follows its problems: norms and
+// step counts, and the run flags (and the sweeps' status) of the latest two
+// GMRES steps, which bgivens writes straight to the host. Pinned memory takes
+// milliseconds to get and to free, so a batch hands its block on: blocks for
+// up to kPollProblems problems go to a list that keeps at most kPollKept of
+// them (4 KB each) and frees the others. A block belongs to one batch at a
+// time, and a batch's solves have ended when it is destroyed.
+constexpr int kPollProblems = 64, kPollKept = 8;
+struct PollBlock {
+  void* mem = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  int device = -1, cap = 0;
+};
+static std::mutex g_poll_mu;
+static std::vector<PollBlock> g_poll_kept;
+
+struct SolvePoll {
+  PollBlock blk;
+  double* norms = nullptr;  // 2 np
+  int* counts = nullptr;    // np
+  int* flags = nullptr;     // 2 (np + 1)
+  cudaEvent_t* ev = blk.ev;
+  SolvePoll() = default;
+  SolvePoll(const SolvePoll&) = delete;
+  SolvePoll& operator=(const SolvePoll&) = delete;
+  int* seen(int step, int np) const { return flags + (size_t)(step & 1) * (np + 1); }
+  static void free_block(PollBlock& b) {
+    for (auto& x : b.ev)
+      if (x) cudaEventDestroy(x);
+    if (b.mem) cudaFreeHost(b.mem);
+    b = PollBlock();
+  }
+  cudaError_t create(int np) {
+    if (blk.mem) return cudaSuccess;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const int cap = std::max(np, kPollProblems);
+    if (cap == kPollProblems) {
+      std::lock_guard<std::mutex> lk(g_poll_mu);
+      for (size_t k = 0; k < g_poll_kept.size(); k++)
+        if (g_poll_kept[k].device == dev) {
+          blk = g_poll_kept[k];
+          g_poll_kept.erase(g_poll_kept.begin() + k);
+          break;
+        }
+    }
+    if (!blk.mem) {
+      blk.device = dev;
+      blk.cap = cap;
+      e = cudaHostAlloc(&blk.mem, sizeof(double) * 2 * cap + sizeof(int) * (3 * (size_t)cap + 2),
+                        cudaHostAllocMapped | cudaHostAllocPortable);
+      for (auto& x : blk.ev)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+      if (e != cudaSuccess) {
+        free_block(blk);
+        return e;
+      }
+    }
+    norms = static_cast<double*>(blk.mem);
+    counts = reinterpret_cast<int*>(norms + 2 * np);
+    flags = counts + np;
+    return cudaSuccess;
+  }
+  ~SolvePoll() {
+    for (auto& x : blk.ev)
+      if (x) cudaEventSynchronize(x);  // no step of an aborted solve writes here any more
+    if (blk.mem && blk.cap == kPollProblems) {
+      std::lock_guard<std::mutex> lk(g_poll_mu);
+      if (g_poll_kept.size() < (size_t)kPollKept) {
+        g_poll_kept.push_back(blk);
+        return;
+      }
+    }
+    free_block(blk);
+  }
+};
+
 struct gf_batch {
   int np = 0, nrows = 0, maxlevL = 0, maxlevU = 0;
   size_t smemL = 0, smemU = 0;  // dynamic shared memory of the level-synchronous sweeps
@@ -2472,9 +2580,10 @@ struct gf_batch {
   DevBuf<int64_t> d_clo, d_chi;
   DevBuf<PermEntry> d_perm_b, d_perm_x, d_perm_out;
   int m = 0;
-  DevBuf<double> V, H, g, cs, ss, y, h, hn, target, partial, pnorm, w, t, r, d, e, norms, bnorm;
+  DevBuf<double> V, H, g, cs, ss, y, hn, target, partial, pnorm, w, t, r, d, e, norms, bnorm;
   DevBuf<double> tfac;
   DevBuf<int> jcnt, run, live, live2;
+  SolvePoll poll;
   gf::BatchAsm* basm = nullptr;  // launch data of the batched assembly
   int scatter = 0;               // 0: coloured, GF_ASSEMBLE_ATOMIC: atomic
   Chunks chunks() const { return Chunks{nchunks, d_cprob.p, d_clo.p, d_chi.p, d_pstart.p}; }
@@ -2775,7 +2884,6 @@ static gf_status ensure_gmres(gf_batch* B, int m) {
   al(B->cs.alloc((size_t)np * m));
   al(B->ss.alloc((size_t)np * m));
   al(B->y.alloc((size_t)np * m));
-  al(B->h.alloc((size_t)np * (m + 1)));
   al(B->hn.alloc(np));
   al(B->target.alloc(np));
   al(B->tfac.alloc(np));
@@ -2789,6 +2897,7 @@ static gf_status ensure_gmres(gf_batch* B, int m) {
   al(B->jcnt.alloc(np));
   al(B->run.alloc(np));
   al(B->live.alloc(np));
+  al(B->poll.create(np));
   if (e != cudaSuccess) {
     set_last_error("gmres workspace", e);
     B->m = 0;
@@ -2800,8 +2909,8 @@ static gf_status ensure_gmres(gf_batch* B, int m) {
 }
 
 static GmArrays arrays(gf_batch* B) {
-  return GmArrays{B->H.p,  B->g.p,      B->cs.p,   B->ss.p,  B->y.p,   B->h.p,
-                  B->hn.p, B->target.p, B->jcnt.p, B->run.p, B->live.p};
+  return GmArrays{B->H.p,      B->g.p,    B->cs.p,  B->ss.p, B->y.p, B->hn.p,
+                  B->target.p, B->jcnt.p, B->run.p, B->live.p};
 }
 
 
@@ -3022,7 +3131,7 @@ static gf_status batch_factor(gf_batch* B, cudaStream_t st) {
 // iters, restarts, rel (true ||b - A x|| / ||b||).
 template <class VT>
 static gf_status bgmres(gf_batch* B, const double* b, double* x, int m, int max_it, double rtol,
-                        int side, int check_every, const std::vector<int>& live0,
+                        int side, const std::vector<int>& live0,
                         std::vector<int>& iters, std::vector<int>& restarts,
                         std::vector<double>& rel, cudaStream_t st) {
   const int np = B->np;
@@ -3032,18 +3141,17 @@ static gf_status bgmres(gf_batch* B, const double* b, double* x, int m, int max_
   const GmArrays G = arrays(B);
   const int nc = B->nchunks;
   const int pb = (np + 127) / 128;
-  std::vector<double> bn(np, 1.0), rn(np);
+  double* const hbn = B->poll.norms;  // host: |b|, then |r| per problem
+  double* const rn = hbn + np;
+  int* const jc = B->poll.counts;
+  std::vector<double> bn(np, 1.0);
   GF_CUDA(cudaMemcpyAsync(B->live.p, live0.data(), sizeof(int) * np, cudaMemcpyHostToDevice, st));
   seg_sumsq<<<nc, kRedThreads, 0, st>>>(b, C, nullptr, B->pnorm.p); ::gf::count_launch();
   seg_norm_out<<<pb, 128, 0, st>>>(B->pnorm.p, C, np, nullptr, B->bnorm.p); ::gf::count_launch();
-  GF_CUDA(cudaMemcpyAsync(bn.data(), B->bnorm.p, sizeof(double) * np, cudaMemcpyDeviceToHost, st));
+  GF_CUDA(cudaMemcpyAsync(hbn, B->bnorm.p, sizeof(double) * np, cudaMemcpyDeviceToHost, st));
   if (side != 0) set_target<<<pb, 128, 0, st>>>(np, B->bnorm.p, rtol, G), ::gf::count_launch();
   GF_CHECK_LAUNCH();
-  GF_CUDA(cudaStreamSynchronize(st));
-  for (int p = 0; p < np; p++)
-    if (bn[p] == 0.0) bn[p] = 1.0;
-  std::vector<int> live = live0, jc(np), runh(np);
-  SweepCtl ctlh{};
+  std::vector<int> live = live0;
   std::vector<double> tf(np, 0.0);
   iters.assign(np, 0);
   restarts.assign(np, 0);
@@ -3057,9 +3165,11 @@ static gf_status bgmres(gf_batch* B, const double* b, double* x, int m, int max_
     if (s != GF_OK) return s;
     seg_sumsq<<<nc, kRedThreads, 0, st>>>(B->r.p, C, B->live.p, B->pnorm.p); ::gf::count_launch();
     seg_norm_out<<<pb, 128, 0, st>>>(B->pnorm.p, C, np, B->live.p, B->norms.p); ::gf::count_launch();
-    GF_CUDA(cudaMemcpyAsync(rn.data(), B->norms.p, sizeof(double) * np, cudaMemcpyDeviceToHost,
-                            st));
+    GF_CUDA(cudaMemcpyAsync(rn, B->norms.p, sizeof(double) * np, cudaMemcpyDeviceToHost, st));
     GF_CUDA(cudaStreamSynchronize(st));
+    if (first)
+      for (int p = 0; p < np; p++)
+        if (hbn[p] != 0.0) bn[p] = hbn[p];
     bool any = false, bad = false;
     for (int p = 0; p < np; p++) {
       if (!live[p]) continue;
@@ -3099,41 +3209,48 @@ static gf_status bgmres(gf_batch* B, const double* b, double* x, int m, int max_
     seg_scale<<<nc, kRedThreads, 0, st>>>(src, B->V.p, C, B->run.p, B->hn.p); ::gf::count_launch();
     GF_CHECK_LAUNCH();
     const int steps = std::min(m, max_it - steps_total);
-    int jj = 0;
-    while (jj < steps) {
-      const int batch = std::min(check_every, steps - jj);
-      for (int k = 0; k < batch; k++, jj++) {
-        const double* vj = B->V.p + (size_t)jj * B->N;
-        if (side == 0) {
-          s = bspmv<VT>(B, B->run.p, vj, 1.0, 0.0, B->t.p, st);
-          if (s == GF_OK) s = bprecond<VT>(B, B->run.p, B->t.p, B->w.p, st);
-        } else {
-          s = bprecond<VT>(B, B->run.p, vj, B->t.p, st);
-          if (s == GF_OK) s = bspmv<VT>(B, B->run.p, B->t.p, 1.0, 0.0, B->w.p, st);
-        }
-        if (s != GF_OK) return s;
-        seg_dots<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, C, B->run.p,
-                                              B->partial.p); ::gf::count_launch();
-        seg_reduce_dots<<<np, 128, 0, st>>>(B->partial.p, C, jj, m, G, 0); ::gf::count_launch();
-        seg_update<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, m, C, G, nullptr); ::gf::count_launch();
-        seg_dots<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, C, B->run.p,
-                                              B->partial.p); ::gf::count_launch();
-        seg_reduce_dots<<<np, 128, 0, st>>>(B->partial.p, C, jj, m, G, 1); ::gf::count_launch();
-        seg_update<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, m, C, G, B->pnorm.p); ::gf::count_launch();
-        seg_norm_finish<<<pb, 128, 0, st>>>(B->pnorm.p, C, np, jj, m, G); ::gf::count_launch();
-        seg_scale<<<nc, kRedThreads, 0, st>>>(B->w.p, B->V.p + (size_t)(jj + 1) * B->N, C,
-                                               B->run.p, B->hn.p); ::gf::count_launch();
-        bgivens<<<pb, 128, 0, st>>>(np, jj, m, steps, G); ::gf::count_launch();
-        GF_CHECK_LAUNCH();
+    for (int jj = 0; jj < steps; jj++) {
+      const double* vj = B->V.p + (size_t)jj * B->N;
+      if (side == 0) {
+        s = bspmv<VT>(B, B->run.p, vj, 1.0, 0.0, B->t.p, st);
+        if (s == GF_OK) s = bprecond<VT>(B, B->run.p, B->t.p, B->w.p, st);
+      } else {
+        s = bprecond<VT>(B, B->run.p, vj, B->t.p, st);
+        if (s == GF_OK) s = bspmv<VT>(B, B->run.p, B->t.p, 1.0, 0.0, B->w.p, st);
       }
-      GF_CUDA(cudaMemcpyAsync(runh.data(), B->run.p, sizeof(int) * np, cudaMemcpyDeviceToHost,
-                              st));
-      GF_CUDA(cudaMemcpyAsync(&ctlh, B->d_ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, st));
-      GF_CUDA(cudaStreamSynchronize(st));
+      if (s != GF_OK) return s;
+      for (int pass = 0; pass < 2; pass++) {  // CGS2
+        seg_dots<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, C, B->run.p, B->partial.p);
+        ::gf::count_launch();
+        seg_update<<<nc, kRedThreads, 0, st>>>(B->V.p, B->w.p, B->N, jj, m, C, G, B->partial.p,
+                                               pass, pass ? B->pnorm.p : nullptr);
+        ::gf::count_launch();
+      }
+      seg_normalize<<<nc, kRedThreads, 0, st>>>(B->w.p, B->V.p + (size_t)(jj + 1) * B->N, C,
+                                                B->run.p, B->pnorm.p);
+      ::gf::count_launch();
+      bgivens<<<(np + 3) / 4, 128, 0, st>>>(np, jj, m, steps, G, B->pnorm.p, C, B->d_ctl.p,
+                                            B->poll.seen(jj, np));
+      ::gf::count_launch();
+      GF_CHECK_LAUNCH();
+      GF_CUDA(cudaEventRecord(B->poll.ev[jj & 1], st));
+      // The step before this one: the GPU keeps a step in hand while the host
+      // launches the next, and at most one step runs after the last problem
+      // has converged (all its kernels return at once). A poll every 25 steps
+      // let a solve of six steps launch 19 such steps: 0.9 ms of 3.3 ms.
+      const int look = jj + 1 < steps ? jj - 1 : jj;
+      if (look < 0) continue;
+      GF_CUDA(cudaEventSynchronize(B->poll.ev[look & 1]));
+      const volatile int* was = B->poll.seen(look, np);
       // a sweep whose bounded wait ran out left a partial z: stop (the
       // caller reads and clears the flag)
-      if (ctlh.status & ST_TIMEOUT) return GF_TIMEOUT;
-      if (std::all_of(runh.begin(), runh.end(), [](int v) { return v == 0; })) break;
+      if (was[np] & ST_TIMEOUT) {
+        GF_CUDA(cudaStreamSynchronize(st));
+        return GF_TIMEOUT;
+      }
+      bool running = false;
+      for (int p = 0; p < np && !running; p++) running = was[p] != 0;
+      if (!running) break;
     }
     bbacksolve<<<pb, 128, 0, st>>>(np, m, G); ::gf::count_launch();
     seg_combine<<<nc, kRedThreads, 0, st>>>(B->V.p, B->N, m, C, G, B->w.p); ::gf::count_launch();
@@ -3146,7 +3263,7 @@ static gf_status bgmres(gf_batch* B, const double* b, double* x, int m, int max_
       seg_axpy<<<nc, kRedThreads, 0, st>>>(1.0, B->w.p, x, C, B->live.p); ::gf::count_launch();
     }
     GF_CHECK_LAUNCH();
-    GF_CUDA(cudaMemcpyAsync(jc.data(), B->jcnt.p, sizeof(int) * np, cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaMemcpyAsync(jc, B->jcnt.p, sizeof(int) * np, cudaMemcpyDeviceToHost, st));
     GF_CUDA(cudaStreamSynchronize(st));
     int mx = 0;
     for (int p = 0; p < np; p++)
@@ -3172,7 +3289,7 @@ static gf_status batch_solve_space(gf_batch* B, const gf_solve_opts& o,
   gf_status result = GF_OK;
   if (!o.mixed) {
     result = bgmres<double>(B, B->d_b.p, B->d_x.p, o.restart, o.max_iters, o.rtol, o.side,
-                            o.check_every, live, iters, rest, rel, st);
+                            live, iters, rest, rel, st);
     for (int p = 0; p < np && !iters.empty(); p++) {
       S[p].iterations = iters[p];
       S[p].restarts = rest[p];
@@ -3238,7 +3355,7 @@ static gf_status batch_solve_space(gf_batch* B, const gf_solve_opts& o,
       // inner solve A32 e = r from zero
       GF_CUDA(cudaMemsetAsync(B->e.p, 0, sizeof(double) * B->N, st));
       s = bgmres<float>(B, B->d.p, B->e.p, o.restart, maxit, o.inner_rtol, o.side,
-                        o.check_every, live, iters, rest, rel, st);
+                        live, iters, rest, rel, st);
       if (s != GF_OK) {
         result = s;
         break;

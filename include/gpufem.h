@@ -339,7 +339,8 @@ typedef struct gf_solve_opts {
                               inner GMRES under FP64 iterative refinement */
   double inner_rtol;      /* inner tolerance per refinement step (mixed) */
   int32_t max_refine;     /* max refinement steps (mixed) */
-  int32_t check_every;    /* host polls convergence every k steps */
+  int32_t check_every;    /* host polls convergence at least every k steps
+                              (it now follows every step, one behind) */
 } gf_solve_opts;
 
 typedef struct gf_solve_stats {
