@@ -142,8 +142,9 @@ constexpr int kMaxEC = 15;
 // distance between a row and a row it multiplies).
 //
 // A triangle solved by the register-fed level sweep (kind TRI_RING) keeps its
-// rows in level order (position p = 0..n-1) too. The kRingWarps warps of a CTA
-// form `groups` groups; group g solves the levels g, g + groups, ... Every
+// rows in level order (position p = 0..n-1) too. The warps of a CTA form
+// `groups` groups of kRingWarps / groups; group g solves the levels g,
+// g + groups, ... Every
 // warp has its own list of passes, tasks[lists[h kRingWarps + warp] ...]: up
 // to 16 blocks of one row a pass, {row (-1: none, -2: the warp helps another
 // one with a long row), blocks | flags | helpers << 5 | rows that the other
@@ -155,7 +156,7 @@ constexpr int kMaxEC = 15;
 // and slots[b] is the ring byte offset of the x entries that block b
 // multiplies. Ring slot 0 holds zeros.
 enum { TRI_LEVEL = 0, TRI_DATAFLOW = 1, TRI_RING = 2 };
-constexpr int kRingWarps = 24;
+constexpr int kRingWarps = 20;  // five a scheduler: 96 registers a thread
 constexpr int kRingCta = 4;  // CTAs of a cluster at most
 constexpr int kRingPad = 4;
 enum {

@@ -1000,14 +1000,17 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
 // the others' rings with st.async, whose bytes their mbarriers count per
 // level (bounded waits; no release of other stores is waited for).
 // Microseconds a level, chunked sweep -> this one (B200): 17x16 plate, ILU(8),
-// FP32 1.19 -> 0.56; 256x128, ILU(6), FP32 2.22 -> 0.85, FP64 3.54 -> 0.89;
-// 250x220, ILU(12), FP32 2.15 -> 0.92; 40x20, complete factor, FP64
-// 1.50 -> 0.58. Still latency-bound: ~120 dependent instructions a level.
+// FP32 1.19 -> 0.46; 256x128, ILU(6), FP32 2.22 -> 0.78, FP64 3.54 -> 0.90;
+// 250x220, ILU(12), FP32 2.15 -> 0.83; 40x20, complete factor, FP64
+// 1.50 -> 0.46. Still latency-bound: ~120 dependent instructions a level, so
+// what the compiler knows to be uniform and what spills shows at once (24
+// warps of 80 registers: 0.51, 0.88, 0.94, 0.91, 0.50; without the broadcast
+// of the warp's number 0.56, 0.85, 0.89, 0.92, 0.58).
 constexpr int kRingThreads = 32 * kRingWarps;
 constexpr size_t kRingSmemMax = 218 * 1024;  // dynamic; the static part is < 1 KB
 // Cost model of a level (clocks; it only chooses the layout), from applies of
 // 17x16 to 250x220 plates, ILU(6) to ILU(12) and complete factors: a chain
-// takes 0.56 us on one CTA and 0.73 us on two or four, a further round of
+// takes 0.5 us on one CTA and 0.7 us on two or four, a further round of
 // passes 0.85 us (its values are not there yet), each pass of a CTA some
 // issue slots; loading and converting hide behind the other groups' levels.
 constexpr double kRingChain = 1000.0, kRingSplit = 350.0, kRingRound = 1700.0, kRingIssue = 70.0,
@@ -1093,7 +1096,10 @@ __global__ void __launch_bounds__(kRingThreads, 1)
   // CTAs without rows leave at once (a cluster barrier counts only threads
   // that have not exited, and no other CTA writes here)
   if ((int)rank >= nsplit) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = lane & 1;
+  // the broadcast tells the compiler that a warp's passes are the same for all
+  // its lanes: no reconvergence around the shuffles of the chain
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int lane = tid & 31, h = lane & 1;
   const bool split = nsplit > 1;
   if (tid == 0) {
     mbar_init(&xbar[0], 1);
@@ -1162,7 +1168,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
   int4 t0 = __ldg(tasks), t1 = __ldg(tasks + 1);
   tasks += 2;
   load(t0);
-  int lev = gi;  // this group's level
+  int lev = gi < groups ? gi : nlev;  // this group's level (a warp beyond the groups has none)
   while (lev < nlev) {
     const int4 t2 = __ldg(tasks++);
     double d[18];
@@ -2357,7 +2363,7 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
   int nsplit = 1, groups = 2;
   double best = 1e300;
   for (int ns = 1; ns <= kRingCta; ns *= 2)
-    for (int g = 2; g <= 3; g++)
+    for (int g = 2; g <= 4; g++)
       if (model(ns, g) < best) {
         best = model(ns, g);
         nsplit = ns;
