@@ -262,11 +262,11 @@ def _dist():
 
 # DRAM bytes (read + write) of a sweep launch over its algorithmic bytes,
 # from an ncu capture of the 256x128 ILU(6) FP32 sweep case (the batch's
-# launches are too large to capture): 85.1 MB / 80.2 MB for L, 89.7 MB /
-# 85.1 MB for U (profiles/bsweep_tma_256x128_ilu6_traffic.md). Traffic per
+# launches are too large to capture): 81.1 MB / 80.2 MB for L, 86.7 MB /
+# 85.1 MB for U (profiles/bsweep_ring_256x128_ilu6.md). Traffic per
 # launch grows with the blocks streamed, so the bench scales the ratio by its
 # own algorithmic bytes per launch.
-SWEEP_TRAFFIC_RATIO = 1.055
+SWEEP_TRAFFIC_RATIO = 1.015
 
 # Fill level k and node ordering of each of the 64 problems, as chosen by the
 # batch autotuner (gpu_fem_b200/batch.py: ordering by ILU(8) levels x blocks
@@ -559,7 +559,7 @@ def main():
     ms_plain = None if args.no_plain else job_ms(plain_fp64_run(bs), ws, "cuda")
 
     # roofline of the dominant kernel, the block triangular sweeps
-    # (bsweep_tma), from CUDA events around every sweep pair inside the timed
+    # (bsweep_ring), from CUDA events around every sweep pair inside the timed
     # mixed-precision region and the algorithmic bytes the sweeps report
     peak, peak_kind = _peaks()
     sweep_s = sweep_ms / 1e3
@@ -589,7 +589,7 @@ def main():
                      "solve": phases_mixed[2]},
         "e2e": {"value": job_throughput(nprob, ws, ms_e2e), "unit": "solves/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": h2d},
-        "roofline": {"kernel": "bsweep_tma (block L and U sweeps, FP32 factor values)",
+        "roofline": {"kernel": "bsweep_ring (block L and U sweeps, FP32 factor values)",
                      "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": SWEEP_TRAFFIC_RATIO * sweep_bytes / max(sweep_launches, 1),

@@ -97,6 +97,10 @@ def factor_work(nrow, inf):
     return nrow * lower * (lower + 1.0)
 
 
+# The cost models below only rank candidates against one another. They were
+# fitted to kernels that took about twice as long as the present ones, sweeps
+# (1.2-2.2 -> 0.46-0.9 us a level) and factorization (9 -> 5 us a level) alike,
+# which leaves the ranking as it is.
 def factor_cost_us(nrow, inf, warps=None):
     """One numeric factorization of a problem (microseconds), fitted to B200
     runs of single plates (16^2 to 256^2 elements, fills 1 to 16) on the
