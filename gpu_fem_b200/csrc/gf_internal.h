@@ -147,9 +147,9 @@ constexpr int kMaxEC = 15;
 // g + groups, ... Every
 // warp has its own list of passes, tasks[lists[h kRingWarps + warp] ...]: up
 // to 16 blocks of one row a pass, {row (-1: none, -2: the warp helps another
-// one with a long row), blocks | flags | helpers << 5 | rows that the other
-// CTAs solve in this level << 16, first block, byte offset of the row's
-// result in the ring (helpers: the warp they help)}. A list ends with
+// one with a long row), blocks | flags | helpers << 5 | 8-byte stores that
+// come from the other CTAs in this level << 16, first block, byte offset of
+// the row's result in the ring (helpers: the warp they help)}. A list ends with
 // kRingPad empty passes. The values of a row's blocks follow each other in
 // `stream` (36 values a block; U rows start with U_ii^{-1}), 16 blocks at a
 // time in the order in which the lanes of a warp load them (ring_value_pos),

@@ -1000,9 +1000,9 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
 // the others' rings with st.async, whose bytes their mbarriers count per
 // level (bounded waits; no release of other stores is waited for).
 // Microseconds a level, chunked sweep -> this one (B200): 17x16 plate, ILU(8),
-// FP32 1.19 -> 0.46; 256x128, ILU(6), FP32 2.22 -> 0.78, FP64 3.54 -> 0.90;
-// 250x220, ILU(12), FP32 2.15 -> 0.83; 40x20, complete factor, FP64
-// 1.50 -> 0.46. Still latency-bound: ~120 dependent instructions a level, so
+// FP32 1.19 -> 0.47; 256x128, ILU(6), FP32 2.22 -> 0.79, FP64 3.54 -> 0.83;
+// 250x220, ILU(12), FP32 2.15 -> 0.82; 40x20, complete factor, FP64
+// 1.50 -> 0.49. Still latency-bound: ~120 dependent instructions a level, so
 // what the compiler knows to be uniform and what spills shows at once (24
 // warps of 80 registers: 0.51, 0.88, 0.94, 0.91, 0.50; without the broadcast
 // of the warp's number 0.56, 0.85, 0.89, 0.92, 0.58).
@@ -1189,7 +1189,7 @@ __global__ void __launch_bounds__(kRingThreads, 1)
         }
       }
       if (split && lead && !abort_flag)
-        mbar_expect_tx(&xbar[lev & 1], 48u * ((unsigned)t0.y >> 16));
+        mbar_expect_tx(&xbar[lev & 1], 8u * ((unsigned)t0.y >> 16));
     }
     if (t0.x != -1) {
       {
@@ -1246,6 +1246,17 @@ __global__ void __launch_bounds__(kRingThreads, 1)
             ob[6 * (size_t)t0.x + rr] = z;
           }
         }
+      }
+    } else if (send && lead && (t0.y & kRingBegin)) {
+      // a CTA without rows in this level says that it has got here (a zero
+      // into slot 0, where a zero is): no CTA solves level l + 1 before every
+      // other one has the results of level l - 1, so bytes of at most two
+      // levels are on their way to a barrier pair, and no ring is written
+      // further ahead than its margin
+      for (int q = 1; q < nsplit; q++) {
+        const unsigned c = (rank + q) & (nsplit - 1);
+        st_async(cluster_map(smem_u32(ring), c), 0.0,
+                 cluster_map(smem_u32(&xbar[lev & 1]), c));
       }
     }
     if (t0.y & kRingEnd) {
@@ -2341,7 +2352,7 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
   // while rows of level l are still being solved the partner may already
   // write rows of level l + 1
   const long long ring = (long long)maxdist + 2ll * maxlev + 1;
-  if ((ring + 1) * 48 > (long long)kRingSmemMax || maxlev > 0xffff) return cudaSuccess;
+  if ((ring + 1) * 48 > (long long)kRingSmemMax || maxlev > 10000) return cudaSuccess;
   auto slot = [&](int i) { return (int)(pos[i] % ring + 1) * 48; };  // slot 0 holds zeros
   // CTAs and groups of warps (clocks on B200): a level costs its chain, a
   // further round for passes beyond one per warp, and the issue slots of its
@@ -2391,7 +2402,10 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
       mine[h].push_back(rows[k]);
     }
     for (int h = 0; h < nsplit; h++) {
-      const int others = ptr[l + 1] - ptr[l] - (int)mine[h].size();
+      // eights of bytes from the other CTAs: six a row, one where there is none
+      int others = 0;
+      for (int q = 0; q < nsplit; q++)
+        if (q != h) others += std::max<int>(1, 6 * (int)mine[q].size());
       const int w0 = h * kRingWarps + (l % groups) * wpg;
       // lists of the group's warps, this level's part
       size_t start[kRingWarps];

@@ -88,3 +88,41 @@ def test_default_sweep_timeout_is_reported():
     P.apply(r, z1)
     assert P.status() == L.GF_OK
     assert torch.equal(z0, z1)
+
+
+@pytest.mark.parametrize("tail", [3, 60])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_default_sweep_levels_of_one_row(tail, precision):
+    """A plate wide enough for a cluster with a strip one element wide at its
+    far corner: the lower sweep ends and the upper one begins with long runs
+    of levels in which only one CTA has a row. Same gate as above."""
+    import torch
+    from gpu_fem_b200.assembler import ElementAssembler, ILUk_Preconditioner, createBsrMat
+    from oracle import pyoracle as po
+    nx, ny = 200, 60
+    m = M.plate(nx, ny + tail, 1.0, 0.3, lambda x, y: 0.006 + 0 * x, "x0",
+                lambda q: 1e3 + 0 * q[:, 0])
+    e = np.arange(m.conn.shape[0])
+    keep = (e // nx < ny) | (e % nx == nx - 1)
+    m.conn, m.thick = m.conn[keep], m.thick[keep]
+    nodes = np.unique(m.conn)
+    new = np.full(m.num_nodes, -1)
+    new[nodes] = np.arange(len(nodes))
+    m.conn, m.xpts = new[m.conn].astype(np.int32), m.xpts[nodes]
+    bcs = m.bcs[new[m.bcs // 6] >= 0]
+    m.bcs = (6 * new[bcs // 6] + bcs % 6).astype(np.int32)
+    A = ElementAssembler.from_mesh(m, ordering="natural")
+    K = createBsrMat(A)
+    A.add_jacobian(None, K, fuse_bcs=True)
+    P = ILUk_Preconditioner(A, 8, precision)
+    P.factor(K)
+    assert P.layout()["nsplit_L"] == 2 and P.layout()["nsplit_U"] == 2
+    rowp, cols, lu = P.get()
+    used = lu.astype(np.float32).astype(np.float64) if precision == "fp32" else lu
+    for seed in range(3):
+        r = np.random.default_rng(seed).standard_normal(m.num_dof)
+        z = torch.full((m.num_dof,), float("nan"), dtype=torch.float64, device="cuda")
+        P.apply(torch.tensor(r, device="cuda"), z)
+        assert P.status() == 0
+        ref = po.ilu_apply_dinv(rowp, cols, used, r)
+        assert np.abs(z.cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
