@@ -67,6 +67,7 @@ struct ChunkSlot {
 // columns (6 bits each), diagonal block, first chunk to touch it, number of
 // contributions.
 enum { kRecColShift = 6, kRecDiag = 1 << 12, kRecFirst = 1 << 13, kRecCountShift = 16 };
+constexpr int kRecMost = 8;  // contributions a record holds, a byte each
 
 // The records of all chunks (brec[bptr[li] ..], nrec[nptr[li] ..] for schedule
 // position li). Host threads take ranges of chunks; within a chunk a small
@@ -98,10 +99,13 @@ static void chunk_records(const gf_mesh_desc& d, const std::vector<int32_t>& ema
         recs.push_back(make_int4(x, info, 0, 0));
       }
       int4& r = recs[start + h[q]];
+      if (first) r.y |= kRecFirst;
+      // an element of four different nodes adds once to a block; one with a
+      // repeated node (no normal there, its entries are NaN) may add more often
       const int n = r.y >> kRecCountShift;
+      if (n == kRecMost) return;
       (n < 4 ? r.z : r.w) |= (int)((unsigned)code << (8 * (n & 3)));
       r.y += 1 << kRecCountShift;
-      if (first) r.y |= kRecFirst;
     };
     for (int li = l0; li < l1; li++) {
       std::memset(at, -1, sizeof(at));
