@@ -1002,19 +1002,24 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
 // Microseconds a level, chunked sweep -> this one (B200): 17x16 plate, ILU(8),
 // FP32 1.19 -> 0.47; 256x128, ILU(6), FP32 2.22 -> 0.79, FP64 3.54 -> 0.83;
 // 250x220, ILU(12), FP32 2.15 -> 0.82; 40x20, complete factor, FP64
-// 1.50 -> 0.49. Still latency-bound: ~120 dependent instructions a level, so
+// 1.50 -> 0.47. Still latency-bound: ~120 dependent instructions a level, so
 // what the compiler knows to be uniform and what spills shows at once (24
 // warps of 80 registers: 0.51, 0.88, 0.94, 0.91, 0.50; without the broadcast
 // of the warp's number 0.56, 0.85, 0.89, 0.92, 0.58).
 constexpr int kRingThreads = 32 * kRingWarps;
 constexpr size_t kRingSmemMax = 218 * 1024;  // dynamic; the static part is < 1 KB
-// Cost model of a level (clocks; it only chooses the layout), from applies of
-// 17x16 to 250x220 plates, ILU(6) to ILU(12) and complete factors: a chain
-// takes 0.5 us on one CTA and 0.7 us on two or four, a further round of
-// passes 0.85 us (its values are not there yet), each pass of a CTA some
-// issue slots; loading and converting hide behind the other groups' levels.
-constexpr double kRingChain = 1000.0, kRingSplit = 350.0, kRingRound = 1700.0, kRingIssue = 70.0,
-                 kRingPrep = 1300.0;
+// Cost model of a level in clocks (it only chooses CTAs and groups): least
+// squares over 300 applies on B200 (22 plates from 17x16 to 256x128, ILU(6) to
+// ILU(12) and complete factors, FP32 and FP64, each with 1, 2, 4 CTAs and 2, 3,
+// 4 groups). Terms: the chain, the exchange of a split, the issue slots of the
+// passes of the busiest CTA, every further round of its busiest warp (a second
+// pass finds its values not there yet), and what the other groups' levels do
+// not hide. Of these layouts it takes the fastest on all plates but one (4 %
+// off). us a level where groups or CTAs decide: 28x28 ILU(12) on one CTA, 2 / 3
+// / 4 groups 0.50 / 0.49 / 0.47; 85x60 ILU(8) on four 0.73 / 0.71 / 0.69;
+// 148x122 ILU(12) on four 0.75 / 0.71 / 1.03 (a second round).
+constexpr double kRingChain = 695.0, kRingSplit = 316.0, kRingSplit4 = 72.0, kRingIssue = 33.0,
+                 kRingRound = 864.0, kRingRoundG = 313.0, kRingLate = 408.0;
 constexpr int kRingAhead = 96 * 1024;  // bytes of values prefetched into L2 ahead of their use
 // rows up to which the chunked level sweep (bsweep_tma) always has a stage:
 // its chunk bound is then the base size of either precision
@@ -2354,32 +2359,65 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
   const long long ring = (long long)maxdist + 2ll * maxlev + 1;
   if ((ring + 1) * 48 > (long long)kRingSmemMax || maxlev > 10000) return cudaSuccess;
   auto slot = [&](int i) { return (int)(pos[i] % ring + 1) * 48; };  // slot 0 holds zeros
-  // CTAs and groups of warps (clocks on B200): a level costs its chain, a
-  // further round for passes beyond one per warp, and the issue slots of its
-  // passes; a split adds the exchange
-  auto model = [&](int ns, int groups) {
-    const int wpg = kRingWarps / groups;
-    double cyc = 0.0;
-    for (int l = 0; l < nlev; l++) {
-      int passes = 0;
-      for (int k = ptr[l]; k < ptr[l + 1]; k++)
-        passes += std::max(1, (end(rows[k]) - beg(rows[k]) + 15) / 16);
-      const int per = (passes + ns - 1) / ns, rounds = (per + wpg - 1) / wpg;
-      const double chain = kRingChain + (upper ? 90.0 : 0.0) + (ns > 1 ? kRingSplit : 0.0) +
-                           kRingRound * (rounds - 1.0) + kRingIssue * per;
-      cyc += std::max(chain, (chain + kRingPrep) / groups);
+  // a level's rows over the CTAs: each to the one with fewer blocks so far
+  // (ties: fewer rows)
+  std::vector<int32_t> mine[kRingCta];
+  auto deal = [&](int l, int ns) {
+    long long hb[kRingCta] = {0};
+    for (auto& m : mine) m.clear();
+    for (int k = ptr[l]; k < ptr[l + 1]; k++) {
+      int h = 0;
+      for (int q = 1; q < ns; q++)
+        if (hb[q] < hb[h] || (hb[q] == hb[h] && mine[q].size() < mine[h].size())) h = q;
+      hb[h] += end(rows[k]) - beg(rows[k]) + first;
+      mine[h].push_back(rows[k]);
     }
-    return cyc;
+  };
+  auto passes = [&](int i) { return std::max(1, (end(i) - beg(i) + 15) / 16); };
+  // warps that share a row of np passes which meets its CTA's warp w with
+  // `left` rows to come: rows are shared while every row still finds warps of
+  // its own (a barrier of helpers is used once a level; the room is 0 or less
+  // once a second round began); the others take their passes one by one
+  auto share = [](int np, int wpg, int w, int left) {
+    return std::max(1, std::min(np, wpg - w - left));
+  };
+  // clocks of all levels on ns CTAs with 2, 3 and 4 groups
+  auto model = [&](int ns, double (&cyc)[5]) {
+    for (int l = 0; l < nlev; l++) {
+      deal(l, ns);
+      for (int g = 2; g <= 4; g++) {
+        const int wpg = kRingWarps / g;
+        int rounds = 1, most = 0;
+        for (int h = 0; h < ns; h++) {
+          int cnt[kRingWarps] = {0}, w = 0, left = (int)mine[h].size(), all = 0;
+          for (int i : mine[h]) {
+            const int np = passes(i), segs = share(np, wpg, w, --left);
+            for (int q = 0; q < segs; q++) {
+              int& c = cnt[w % wpg + q];
+              rounds = std::max(rounds, c += np * (q + 1) / segs - np * q / segs);
+            }
+            w += segs;
+            all += np;
+          }
+          most = std::max(most, all);
+        }
+        cyc[g] += kRingChain + (ns > 1 ? kRingSplit : 0.0) + (ns > 2 ? kRingSplit4 : 0.0) +
+                  kRingIssue * most + (rounds - 1) * (kRingRound + kRingRoundG / g) + kRingLate / g;
+      }
+    }
   };
   int nsplit = 1, groups = 2;
   double best = 1e300;
-  for (int ns = 1; ns <= kRingCta; ns *= 2)
+  for (int ns = 1; ns <= kRingCta; ns *= 2) {
+    double cyc[5] = {0.0};
+    model(ns, cyc);
     for (int g = 2; g <= 4; g++)
-      if (model(ns, g) < best) {
-        best = model(ns, g);
+      if (cyc[g] < best) {
+        best = cyc[g];
         nsplit = ns;
         groups = g;
       }
+  }
   const int wpg = kRingWarps / groups;
   size_t nblocks = (size_t)first * n;
   for (int i = 0; i < n; i++) nblocks += end(i) - beg(i);
@@ -2387,20 +2425,9 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
   std::vector<uint16_t> code(nblocks);
   std::vector<std::vector<int4>> lists((size_t)kRingCta * kRingWarps);
   size_t b = 0;
-  std::vector<int32_t> mine[kRingCta];
   long long npass = 0;
   for (int l = 0; l < nlev; l++) {
-    // a level's rows over the CTAs: each to the one with fewer blocks so far
-    // (ties: fewer rows)
-    long long hb[kRingCta] = {0};
-    for (auto& m : mine) m.clear();
-    for (int k = ptr[l]; k < ptr[l + 1]; k++) {
-      int h = 0;
-      for (int q = 1; q < nsplit; q++)
-        if (hb[q] < hb[h] || (hb[q] == hb[h] && mine[q].size() < mine[h].size())) h = q;
-      hb[h] += end(rows[k]) - beg(rows[k]) + first;
-      mine[h].push_back(rows[k]);
-    }
+    deal(l, nsplit);
     for (int h = 0; h < nsplit; h++) {
       // eights of bytes from the other CTAs: six a row, one where there is none
       int others = 0;
@@ -2410,15 +2437,10 @@ static cudaError_t build_ring(gf_precond* p, const std::vector<int32_t>& diag, b
       // lists of the group's warps, this level's part
       size_t start[kRingWarps];
       for (int w = 0; w < wpg; w++) start[w] = lists[w0 + w].size();
-      // rows of several passes are shared while every row still finds warps
-      // of its own (a barrier of helpers is used once a level); the others
-      // take their passes one after another
       int w = 0, left = (int)mine[h].size();
       for (int i : mine[h]) {
-        const int nb = end(i) - beg(i), np = std::max(1, (nb + 15) / 16);
-        left--;
-        const int room = wpg - w - left;  // 0 or less once a second round began
-        const int segs = std::max(1, std::min(np, room));
+        const int nb = end(i) - beg(i), np = passes(i);
+        const int segs = share(np, wpg, w, --left);
         int pass = 0;
         for (int q = 0; q < segs; q++) {
           auto& L = lists[w0 + w % wpg + q];
