@@ -43,6 +43,8 @@ constexpr int kRedThreads = 256;
 struct SweepCtl {
   int status;
   int pivot;
+  int gave_up, quiet;  // CTAs of split ring sweeps whose wait ran out; those of them that left
+                       // with no store in flight to them
 };
 
 // ------------------------------------------------ barriers and bulk copies
@@ -998,16 +1000,21 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
 //  - rows of more than 16 blocks are shared by several warps.
 // In a triangle split over the CTAs of a cluster every result also goes to
 // the others' rings with st.async, whose bytes their mbarriers count per
-// level (bounded waits; no release of other stores is waited for).
-// Microseconds a level, chunked sweep -> this one (B200): 17x16 plate, ILU(8),
-// FP32 1.19 -> 0.47; 256x128, ILU(6), FP32 2.22 -> 0.79, FP64 3.54 -> 0.83;
-// 250x220, ILU(12), FP32 2.15 -> 0.82; 40x20, complete factor, FP64
-// 1.50 -> 0.47. Still latency-bound: ~120 dependent instructions a level, so
-// what the compiler knows to be uniform and what spills shows at once (24
-// warps of 80 registers: 0.51, 0.88, 0.94, 0.91, 0.50; without the broadcast
+// level (bounded waits; no release of other stores is waited for). A warp
+// whose wait runs out solves, arms and sends nothing from that level on, nor
+// does any warp of its CTA from the next level on (ring_leave), so no barrier
+// ever counts the bytes of more than two levels (below the 2^20 - 1 that it
+// can); the CTA ends once the bytes that were sent to it have landed
+// (ring_drain). Microseconds a level, chunked sweep -> this one (B200): 17x16
+// plate, ILU(8), FP32 1.19 -> 0.45; 256x128, ILU(6), FP32 2.22 -> 0.76, FP64
+// 3.54 -> 0.79; 250x220, ILU(12), FP32 2.15 -> 0.83; 40x20, complete factor,
+// FP64 1.50 -> 0.47. Still latency-bound: ~120 dependent instructions a level,
+// so what the compiler knows to be uniform and what spills shows at once (with
+// one body for split and unsplit triangles 0.47, 0.79, 0.83, 0.82, 0.47; then
+// with 24 warps of 80 registers 0.51, 0.88, 0.94, 0.91, 0.50; without the broadcast
 // of the warp's number 0.56, 0.85, 0.89, 0.92, 0.58).
 constexpr int kRingThreads = 32 * kRingWarps;
-constexpr size_t kRingSmemMax = 218 * 1024;  // dynamic; the static part is < 1 KB
+constexpr size_t kRingSmemMax = 218 * 1024;  // dynamic; the static part is < 2 KB
 // Cost model of a level in clocks (it only chooses CTAs and groups): least
 // squares over 300 applies on B200 (22 plates from 17x16 to 256x128, ILU(6) to
 // ILU(12) and complete factors, FP32 and FP64, each with 1, 2, 4 CTAs and 2, 3,
@@ -1081,31 +1088,121 @@ __device__ __forceinline__ void ring_take(const double (&v)[18], double (&d)[18]
   for (int k = 0; k < 18; k++) d[k] = v[k];
 }
 
-template <class VT, bool UPPER>
-__global__ void __launch_bounds__(kRingThreads, 1)
-    bsweep_ring(const ProbDev* __restrict__ P, const int* __restrict__ live,
-                const double* __restrict__ rhs, double* out, SweepCtl* ctl,
-                unsigned long long* bytes_ctr) {
-  extern __shared__ __align__(128) unsigned char ring[];
-  __shared__ uint64_t xbar[2];  // the other CTAs' results of even / odd levels
-  __shared__ double part[kRingWarps][6];  // a helper's sums for the row's warp
-  __shared__ volatile int abort_flag;
-  unsigned ncta;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
-  const int p = blockIdx.x / ncta;
-  const unsigned rank = cluster_rank();
-  if (live && !live[p]) return;  // the same for every CTA of the cluster
-  const TriDesc& T = UPPER ? P[p].U : P[p].L;
-  if (T.kind != TRI_RING) return;
-  const int nsplit = T.nsplit;
-  // CTAs without rows leave at once (a cluster barrier counts only threads
-  // that have not exited, and no other CTA writes here)
-  if ((int)rank >= nsplit) return;
+// Waits (bounded) until a phase of bar is complete, as one warp: false when
+// the bound ran out (abort_flag set here) or another warp's did. That comes
+// first: past a level in which a warp gave up, a barrier may be a phase behind,
+// and its parity then reads as complete.
+__device__ __noinline__ bool ring_wait(uint64_t* bar, unsigned parity,
+                                       volatile int* abort_flag) {
+  const unsigned long long t0 = gtimer();
+  while (true) {
+    if (__any_sync(0xffffffffu, *abort_flag)) return false;
+    if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, gtimer() - t0 > g_wait_ns)) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+}
+
+// The rest of a warp's levels after it has given up in level lev (pass t, whose
+// barrier it has met): it only meets the barriers that other warps wait at.
+__device__ __noinline__ void ring_leave(const int4* t, int lev, int nlev, int groups, int warp) {
+  const int wpg = kRingWarps / groups, gi = warp / wpg, bar_threads = 64 * wpg;
+  const int bar_in = 1 + (gi ? gi - 1 : groups - 1), bar_out = 1 + gi;
+  for (bool met = true; lev < nlev; met = false) {
+    const int4 k = __ldg(t++);
+    if ((k.y & kRingBegin) && !met) named_sync(bar_in, bar_threads);
+    const int helpers = (k.y >> 5) & 31;
+    if (k.y & kRingLast) {
+      if (k.x == -2)
+        named_arrive((1 + groups + k.w / 2) & 15, 32 * (helpers + 1));
+      else if (helpers)
+        named_sync((1 + groups + warp / 2) & 15, 32 * (helpers + 1));
+    }
+    if (k.y & kRingEnd) {
+      if (lev + 1 < nlev) named_arrive(bar_out, bar_threads);
+      lev += groups;
+    }
+  }
+}
+
+// A CTA that gave up waits here (bounded) for the stores that are still on
+// their way into it; nothing is sent to it any more. gone[q][w] is the level
+// in which warp w of CTA q gave up: it armed and sent nothing from there on.
+// The bytes sent to this CTA and the bytes its barriers were armed for follow
+// from the task lists; where they differ the last phase's count is set right,
+// so that it completes with the last byte.
+__device__ __noinline__ void ring_drain(const TriDesc& T, unsigned rank,
+                                        const int (*gone)[kRingWarps], uint64_t* xbar,
+                                        SweepCtl* ctl) {
+  __shared__ int armed[2], sent[2], arms[2];  // bytes, bytes, phases of even / odd levels
+  const int tid = threadIdx.x;
+  if (tid < 2) armed[tid] = sent[tid] = arms[tid] = 0;
+  __syncthreads();
+  if (tid < T.nsplit * kRingWarps) {
+    const int q = tid / kRingWarps, w = tid % kRingWarps, wpg = kRingWarps / T.groups;
+    const bool lead = w % wpg == 0, mine = q == (int)rank;
+    const int end = min(T.nlev, gone[q][w]);
+    const int4* t = T.tasks + T.lists[q * kRingWarps + w];
+    int lev = w / wpg < T.groups ? w / wpg : T.nlev;
+    for (; lev < end; t++) {
+      const int4 k = *t;
+      if (mine) {
+        if (lead && (k.y & kRingBegin)) {
+          atomicAdd(&armed[lev & 1], 8 * (int)((unsigned)k.y >> 16));
+          atomicAdd(&arms[lev & 1], 1);
+        }
+      } else if (k.x >= 0 ? (k.y & kRingLast) : (k.x == -1 && lead && (k.y & kRingBegin))) {
+        atomicAdd(&sent[lev & 1], k.x >= 0 ? 48 : 8);
+      }
+      if (k.y & kRingEnd) lev += T.groups;
+    }
+  }
+  __syncthreads();
+  if (tid != 0) return;
+  bool quiet = true;
+  for (int z = 0; z < 2; z++) {
+    const int more = sent[z] - armed[z];
+    if (more < 0)
+      asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(
+                       smem_u32(&xbar[z])),
+                   "r"(-more)
+                   : "memory");
+    if (arms[z] > 0)
+      quiet &= mbar_wait_cluster(&xbar[z], (unsigned)((arms[z] - 1) & 1), kWaitNs);
+    if (more > 0 && quiet) {
+      mbar_expect_tx(&xbar[z], (unsigned)more);
+      quiet &= mbar_wait_cluster(&xbar[z], (unsigned)(arms[z] & 1), kWaitNs);
+    }
+  }
+  atomicOr(&ctl->status, ST_TIMEOUT);
+  atomicAdd(&ctl->gave_up, 1);
+  if (quiet) atomicAdd(&ctl->quiet, 1);
+}
+
+struct RingShared {
+  uint64_t xbar[2];            // the other CTAs' results of even / odd levels
+  double part[kRingWarps][6];  // a helper's sums for the row's warp
+  int gone[kRingCta][kRingWarps];  // per CTA and warp: level in which it gave up (ring_drain)
+  volatile int abort_flag;         // a warp of this CTA has
+};
+
+// The sweep of one triangle; SPLIT: shared by the CTAs of a cluster. (In one
+// body for both, what a split needs costs an unsplit level too: 33x21 plate,
+// ILU(8), FP64 0.55 us instead of 0.52.)
+template <class VT, bool UPPER, bool SPLIT>
+__device__ __forceinline__ void ring_sweep(unsigned char* ring, RingShared& sh, const TriDesc& T,
+                                           int nsplit, unsigned rank, const double* rb, double* ob,
+                                           SweepCtl* ctl, unsigned long long* bytes_ctr) {
+  uint64_t* xbar = sh.xbar;
+  auto part = sh.part;
+  auto gone = sh.gone;
+  volatile int& abort_flag = sh.abort_flag;
   // the broadcast tells the compiler that a warp's passes are the same for all
   // its lanes: no reconvergence around the shuffles of the chain
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31, h = lane & 1;
-  const bool split = nsplit > 1;
   if (tid == 0) {
     mbar_init(&xbar[0], 1);
     mbar_init(&xbar[1], 1);
@@ -1113,13 +1210,13 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     abort_flag = 0;
   }
   if (tid < 6) reinterpret_cast<double*>(ring)[tid] = 0.0;
-  if (split)
+  if (tid < kRingCta * kRingWarps) gone[0][tid] = 0x7fffffff;
+  if (SPLIT)
     cluster_barrier();  // every CTA's barriers exist before any remote store
   else
     __syncthreads();
-  const bool send = split && !(g_skip_meet && rank == 1);
-  const double* rb = rhs + 6 * (size_t)P[p].off;
-  double* ob = out + 6 * (size_t)P[p].off;
+  const bool mute = g_skip_meet && rank == 1;  // failure injection
+  const int peers = SPLIT && !mute ? nsplit : 0;
   const unsigned char* stream = T.stream;
   const VT* vals = reinterpret_cast<const VT*>(stream);
   const int32_t* slots = T.slots;
@@ -1182,19 +1279,18 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     if (t0.y & kRingBegin) {
       if (lev > 0) {
         named_sync(bar_in, bar_threads);
-        if (split && !abort_flag) {
+        if (SPLIT) {  // the results of the other CTAs, as one warp
           uint64_t* b = &xbar[(lev - 1) & 1];
           const unsigned par = (unsigned)(((lev - 1) >> 1) & 1);
-          unsigned long long w0 = 0;
-          while (!mbar_try_wait_cluster(b, par)) {
-            if (abort_flag) break;
-            if (w0 == 0) w0 = gtimer();
-            if (gtimer() - w0 > g_wait_ns) abort_flag = 1;
+          const int quit = abort_flag;  // a warp has given up, here or in a level before
+          if (!__all_sync(0xffffffffu, mbar_try_wait_cluster(b, par) && !quit) &&
+              !__all_sync(0xffffffffu, ring_wait(b, par, &abort_flag))) {
+            if (lane == 0) gone[rank][warp] = lev;
+            ring_leave(tasks - 3, lev, nlev, groups, warp);
+            break;
           }
         }
       }
-      if (split && lead && !abort_flag)
-        mbar_expect_tx(&xbar[lev & 1], 8u * ((unsigned)t0.y >> 16));
     }
     if (t0.x != -1) {
       {
@@ -1242,9 +1338,11 @@ __global__ void __launch_bounds__(kRingThreads, 1)
           if (writer) {
             const unsigned o = (unsigned)t0.w + 8u * (unsigned)rr;
             *reinterpret_cast<double*>(ring + o) = z;
-            if (send)
-              for (int q = 1; q < nsplit; q++) {
-                const unsigned c = (rank + q) & (nsplit - 1);
+            if (SPLIT)
+#pragma unroll
+              for (int q = 1; q < kRingCta; q++) {
+                if (q >= peers) break;
+                const unsigned c = rank ^ q;
                 st_async(cluster_map(smem_u32(ring + o), c), z,
                          cluster_map(smem_u32(&xbar[lev & 1]), c));
               }
@@ -1252,18 +1350,22 @@ __global__ void __launch_bounds__(kRingThreads, 1)
           }
         }
       }
-    } else if (send && lead && (t0.y & kRingBegin)) {
+    } else if (SPLIT && lead && (t0.y & kRingBegin)) {
       // a CTA without rows in this level says that it has got here (a zero
       // into slot 0, where a zero is): no CTA solves level l + 1 before every
       // other one has the results of level l - 1, so bytes of at most two
       // levels are on their way to a barrier pair, and no ring is written
       // further ahead than its margin
-      for (int q = 1; q < nsplit; q++) {
-        const unsigned c = (rank + q) & (nsplit - 1);
+      for (int q = 1; q < peers; q++) {
+        const unsigned c = rank ^ q;
         st_async(cluster_map(smem_u32(ring), c), 0.0,
                  cluster_map(smem_u32(&xbar[lev & 1]), c));
       }
     }
+    // bytes of this level may have landed before; arming after the pass keeps
+    // it off the chain (85x60, ILU(8), FP32 0.65 -> 0.63 us a level)
+    if (SPLIT && lead && (t0.y & kRingBegin))
+      mbar_expect_tx(&xbar[lev & 1], 8u * ((unsigned)t0.y >> 16));
     if (t0.y & kRingEnd) {
       if (lev + 1 < nlev) named_arrive(bar_out, bar_threads);
       lev += groups;
@@ -1272,23 +1374,54 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     t1 = t2;
     load(t0);
   }
-  if (split) {
-    // the other CTAs' results of the last level have landed (nothing may
-    // be in flight into a CTA that ends)
+  if (SPLIT) {
+    // the other CTAs' results of the last level have landed
     __syncthreads();
     if (tid == 0 && !abort_flag &&
         !mbar_wait_cluster(&xbar[(nlev - 1) & 1], (unsigned)(((nlev - 1) >> 1) & 1), g_wait_ns))
       abort_flag = 1;
-    if (tid == 0 && abort_flag) atomicOr(&ctl->status, ST_TIMEOUT);
+    __syncthreads();
+    if ((abort_flag || mute) && tid < kRingWarps)
+      for (int q = 1; q < nsplit; q++)
+        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_map(
+                         smem_u32(&gone[rank][tid]), rank ^ q)),
+                     "r"(mute ? 0 : gone[rank][tid])
+                     : "memory");
   }
   if (tid == 0 && rank == 0 && bytes_ctr && !abort_flag)
     atomicAdd(bytes_ctr, (unsigned long long)T.abytes);
-  if (split) {
-    // no CTA leaves while another may still write into its ring; every path
-    // of every CTA of a split problem reaches this point
-    __syncthreads();
+  if (SPLIT) {
+    // From here on nobody sends. A CTA that has not given up has waited for
+    // every byte of every level; one that has waits for what it was sent.
     cluster_barrier();
+    if (abort_flag) ring_drain(T, rank, gone, xbar, ctl);
   }
+}
+
+template <class VT, bool UPPER>
+__global__ void __launch_bounds__(kRingThreads, 1)
+    bsweep_ring(const ProbDev* __restrict__ P, const int* __restrict__ live,
+                const double* __restrict__ rhs, double* out, SweepCtl* ctl,
+                unsigned long long* bytes_ctr) {
+  extern __shared__ __align__(128) unsigned char ring[];
+  __shared__ RingShared sh;
+  unsigned ncta;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+  const int p = blockIdx.x / ncta;
+  const unsigned rank = cluster_rank();
+  if (live && !live[p]) return;  // the same for every CTA of the cluster
+  const TriDesc& T = UPPER ? P[p].U : P[p].L;
+  if (T.kind != TRI_RING) return;
+  const int nsplit = T.nsplit;
+  // CTAs without rows leave at once (a cluster barrier counts only threads
+  // that have not exited, and no other CTA writes here)
+  if ((int)rank >= nsplit) return;
+  const double* rb = rhs + 6 * (size_t)P[p].off;
+  double* ob = out + 6 * (size_t)P[p].off;
+  if (nsplit > 1)
+    ring_sweep<VT, UPPER, true>(ring, sh, T, nsplit, rank, rb, ob, ctl, bytes_ctr);
+  else
+    ring_sweep<VT, UPPER, false>(ring, sh, T, 1, 0, rb, ob, ctl, bytes_ctr);
 }
 
 // Factor values into a ring sweep's stream: block q of the triangle takes
@@ -2613,6 +2746,7 @@ struct gf_batch {
   DevBuf<ProbDev> d_desc;
   DevBuf<int32_t> d_row_prob;
   DevBuf<SweepCtl> d_ctl;
+  int gave_up = 0, quiet = 0;        // SweepCtl's, when it was last read
   DevBuf<double> d_tmp, d_b, d_x;
   int nchunks = 0;
   DevBuf<int32_t> d_cprob, d_pstart;
@@ -3092,6 +3226,8 @@ static gf_status read_ctl(gf_batch* B, cudaStream_t st, SweepCtl* h) {
   GF_CUDA(cudaMemcpyAsync(h, B->d_ctl.p, sizeof(SweepCtl), cudaMemcpyDeviceToHost, st));
   GF_CUDA(cudaMemsetAsync(B->d_ctl.p, 0, sizeof(SweepCtl), st));
   GF_CUDA(cudaStreamSynchronize(st));
+  B->gave_up = h->gave_up;
+  B->quiet = h->quiet;
   return GF_OK;
 }
 static gf_status ctl_status(const SweepCtl& h) {
@@ -3674,6 +3810,13 @@ gf_status gf_test_set_waits(unsigned long long wait_ns, int32_t skip_meetings) {
   const int k = skip_meetings ? 1 : 0;
   GF_CUDA(cudaMemcpyToSymbol(g_wait_ns, &w, sizeof(w)));
   GF_CUDA(cudaMemcpyToSymbol(g_skip_meet, &k, sizeof(k)));
+  return GF_OK;
+}
+
+gf_status gf_test_sweep_exits(const gf_precond* p, int32_t* gave_up, int32_t* quiet) {
+  if (!p) return GF_INVALID_ARG;
+  if (gave_up) *gave_up = p->self ? p->self->gave_up : 0;
+  if (quiet) *quiet = p->self ? p->self->quiet : 0;
   return GF_OK;
 }
 

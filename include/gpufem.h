@@ -426,11 +426,17 @@ gf_status gf_batch_solve(gf_batch* b, const double* const* d_b, double* const* d
  * never publishes the first row of its order and the dataflow sweep's warp
  * 0 never publishes its rows, which makes the bounded waits run out so that
  * the launch reports GF_TIMEOUT. The waits that drain a CTA's own copies
- * in flight keep the 2 s bound, and both CTAs of a cluster still meet on the
- * final cluster barrier, so nothing hangs. Process-wide for the device: set
+ * in flight (and, in the default sweep, the stores in flight to it) keep the
+ * 2 s bound, and all CTAs of a cluster still meet on the final cluster
+ * barrier, so nothing hangs. Process-wide for the device: set
  * it only while no other work of this library runs there, and restore it
  * with gf_test_set_waits(0, 0). No reference counterpart. */
 gf_status gf_test_set_waits(unsigned long long wait_ns, int32_t skip_meetings);
+/* Of the sweeps between the last two reads of the preconditioner's device
+ * status (gf_precond_status): CTAs of split default sweeps that gave up
+ * waiting, and those of them that left with no store in flight to them (all
+ * of them, or the kernel is wrong). No reference counterpart. */
+gf_status gf_test_sweep_exits(const gf_precond* p, int32_t* gave_up, int32_t* quiet);
 
 #ifdef __cplusplus
 }
