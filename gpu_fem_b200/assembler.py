@@ -399,6 +399,13 @@ class ILUk_Preconditioner:
         return {"nsplit_L": v[0].value, "nsplit_U": v[1].value, "fac_ctas": v[2].value,
                 "chunks_L": v[3].value, "chunks_U": v[4].value}
 
+    def factor_layout(self):
+        """Rows whose values / whose column -> slot map the factorization keeps
+        in shared memory (gf_precond_factor_layout)."""
+        s, m = C.c_int32(), C.c_int32()
+        check(L.lib().gf_precond_factor_layout(self.h, C.byref(s), C.byref(m)), "factor_layout")
+        return {"staged": s.value, "mapped": m.value}
+
     def setup_info(self):
         """gf_precond_setup_info: whether the ILU(k) pattern was computed on
         the GPU, and the host wall times (ms) of the pattern and the setup."""

@@ -319,6 +319,11 @@ gf_status gf_precond_setup_info(const gf_precond* p, int32_t* symbolic_on_gpu, d
                                 double* setup_ms);
 gf_status gf_precond_layout(const gf_precond* p, int32_t* nsplit_L, int32_t* nsplit_U,
                             int32_t* fac_ctas, int32_t* chunks_L, int32_t* chunks_U);
+/* Rows of the factor whose values (at most 80 blocks) and whose column -> slot
+ * map (at most 1024 columns from the first to the last) the factorization
+ * keeps in shared memory; the others are updated, or searched, in global
+ * memory. Any pointer may be NULL. No reference counterpart. */
+gf_status gf_precond_factor_layout(const gf_precond* p, int32_t* staged, int32_t* mapped);
 /* Pattern, level count and factor copy for checking. rowPtr/colPtr may be
  * NULL; values receives nnzb_pc*36 entries with the diagonal blocks holding
  * U_ii^{-1}. */
