@@ -213,6 +213,13 @@ class ElementAssembler:
         check(L.lib().gf_assembler_setup_info(self.h, C.byref(p), C.byref(m)), "setup_info")
         return {"pattern_on_gpu": bool(p.value), "elem_map_on_gpu": bool(m.value)}
 
+    def setup_times(self):
+        """gf_assembler_setup_times: wall times (ms) of the whole setup and of
+        the chunk records in it."""
+        r, t = C.c_double(), C.c_double()
+        check(L.lib().gf_assembler_setup_times(self.h, C.byref(r), C.byref(t)), "setup_times")
+        return {"records_ms": r.value, "setup_ms": t.value}
+
     def tune_scatter(self, mat, reps=5):
         """Times the Jacobian with the coloured and the atomic scatter on
         `mat` and keeps the faster for add_jacobian(atomic=None); returns the

@@ -41,13 +41,17 @@
 // wavefronts (l1tex 62 %, FP64 pipe 20 %, 15 warps an SM), the residual by
 // instruction latency (FP64 pipe 28 %).
 #include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
-#include <thread>
 
 #include "gf_internal.h"
 
 namespace gf {
+
+static double ms_since(std::chrono::steady_clock::time_point t) {
+  return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count();
+}
 
 constexpr int kChunkSize = 8;     // elements per chunk
 constexpr int kAsmThreads = 128;  // a warp takes every fourth element
@@ -68,77 +72,110 @@ struct ChunkSlot {
 // contributions.
 enum { kRecColShift = 6, kRecDiag = 1 << 12, kRecFirst = 1 << 13, kRecCountShift = 16 };
 constexpr int kRecMost = 8;  // contributions a record holds, a byte each
+// an element has four different nodes, so it adds at most once to a block
+static_assert(kChunkSize <= kRecMost, "a chunk's contributions to a block fit its record");
 
-// The records of all chunks (brec[bptr[li] ..], nrec[nptr[li] ..] for schedule
-// position li). Host threads take ranges of chunks; within a chunk a small
-// hash table finds the record of a block or node.
-static void chunk_records(const gf_mesh_desc& d, const std::vector<int32_t>& emap,
-                          const Schedule& s, const std::vector<uint8_t>& bcmask,
-                          std::vector<int4>& brec, std::vector<int32_t>& bptr,
-                          std::vector<int4>& nrec, std::vector<int32_t>& nptr) {
-  constexpr int kHash = 256;  // twice the records a chunk can have
-  const int nt = s.nchunks < 256 ? 1 : (int)std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-  struct Part {
-    std::vector<int4> brec, nrec;
-  };
-  std::vector<Part> parts(nt);
-  bptr.assign(s.nchunks + 1, 0);
-  nptr.assign(s.nchunks + 1, 0);
-  auto work = [&](int t) {
-    Part& part = parts[t];
-    const int l0 = (int)((long long)s.nchunks * t / nt), l1 = (int)((long long)s.nchunks * (t + 1) / nt);
-    part.brec.reserve((size_t)80 * (l1 - l0) + 128);
-    part.nrec.reserve((size_t)17 * (l1 - l0) + 32);
-    int16_t at[2][kHash];
-    auto add = [&](std::vector<int4>& recs, int16_t* h, size_t start, int x, int info, int code,
-                   bool first) {
-      int q = (int)(((unsigned)x * 2654435761u) >> 24);
-      while (h[q] >= 0 && recs[start + h[q]].x != x) q = (q + 1) & (kHash - 1);
-      if (h[q] < 0) {
-        h[q] = (int16_t)(recs.size() - start);
-        recs.push_back(make_int4(x, info, 0, 0));
-      }
-      int4& r = recs[start + h[q]];
-      if (first) r.y |= kRecFirst;
-      // an element of four different nodes adds once to a block; one with a
-      // repeated node (no normal there, its entries are NaN) may add more often
-      const int n = r.y >> kRecCountShift;
-      if (n == kRecMost) return;
-      (n < 4 ? r.z : r.w) |= (int)((unsigned)code << (8 * (n & 3)));
-      r.y += 1 << kRecCountShift;
-    };
-    for (int li = l0; li < l1; li++) {
-      std::memset(at, -1, sizeof(at));
-      const size_t b0 = part.brec.size(), n0 = part.nrec.size();
-      for (int q = s.chunk_start[li]; q < s.chunk_start[li + 1]; q++) {
-        const int e = s.order[q], k = q - s.chunk_start[li];
-        for (int x = 0; x < 4; x++) {
-          const int na = d.conn[4 * e + x];
-          add(part.nrec, at[1], n0, na, bcmask[na], 4 * k + x, (s.first_touch[e] >> (16 + x)) & 1);
-          for (int y = 0; y < 4; y++)
-            add(part.brec, at[0], b0, emap[16 * e + 4 * x + y],
-                bcmask[na] | bcmask[d.conn[4 * e + y]] << kRecColShift | (x == y ? kRecDiag : 0),
-                16 * k + 4 * x + y, (s.first_touch[e] >> (4 * x + y)) & 1);
-        }
-      }
-      bptr[li + 1] = (int32_t)(part.brec.size() - b0);
-      nptr[li + 1] = (int32_t)(part.nrec.size() - n0);
+// Records of chunk blockIdx.x, in the order of their first contributions (recs
+// null: their numbers only, blocks | nodes << 16 in count). A thread a
+// contribution: 16 blocks an element, then 4 nodes. Built on the host (a hash
+// table a chunk) the records were half of an assembler's setup: 400x200 plate
+// 19 of 37 ms, now 1.7 of 24, most of it the upload of the elemIndMap; 10x10
+// 0.06 -> 0.09 ms (two launches and a read-back).
+__global__ void __launch_bounds__(16 * kChunkSize)
+    chunk_records_kernel(const int32_t* __restrict__ chunk_start, const int32_t* __restrict__ order,
+                         const int32_t* __restrict__ sconn, const int32_t* __restrict__ emap,
+                         const uint32_t* __restrict__ first_touch,
+                         const uint8_t* __restrict__ bcmask, const int32_t* __restrict__ ptr,
+                         int32_t* __restrict__ count, int4* __restrict__ recs) {
+  constexpr int T = 16 * kChunkSize;
+  __shared__ int key[2][T];             // block or node of each contribution
+  __shared__ unsigned char touch[2][T];  // first chunk to touch it
+  __shared__ int warps[T / 32];
+  const int li = blockIdx.x, t = threadIdx.x, lane = t & 31;
+  const int s0 = chunk_start[li], cnt = chunk_start[li + 1] - s0;
+  for (int z = 0; z < 2; z++) {  // blocks, nodes
+    const int per = z ? 4 : 16, k = t / per, x = t % per;
+    const bool on = k < cnt;
+    const int e = on ? order[s0 + k] : 0;
+    key[z][t] = !on ? -1 : z ? sconn[4 * (s0 + k) + x] : emap[16 * (size_t)e + x];
+    touch[z][t] = on ? (first_touch[e] >> (16 * z + x)) & 1 : 0;
+  }
+  __syncthreads();
+  for (int z = 0; z < 2; z++) {
+    const int n = (z ? 4 : 16) * cnt, mine = key[z][t];
+    bool first = t < n;
+    for (int j = 0; j < t && j < n; j++) first = first && key[z][j] != mine;
+    const unsigned vote = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) warps[t >> 5] = __popc(vote);
+    __syncthreads();
+    int at = __popc(vote & ((1u << lane) - 1u)), all = 0;
+    for (int w = 0; w < T / 32; w++) {
+      if (w < t >> 5) at += warps[w];
+      all += warps[w];
     }
+    __syncthreads();
+    if (!recs) {
+      if (t == 0) count[li] = z ? count[li] | all << 16 : all;
+      continue;
+    }
+    if (!first) continue;
+    const int a = z ? mine : sconn[4 * s0 + t / 4], b = z ? a : sconn[4 * (s0 + t / 16) + t % 4];
+    int4 r = make_int4(mine, bcmask[a], 0, 0);
+    if (!z) r.y |= bcmask[b] << kRecColShift | (a == b ? kRecDiag : 0);
+    int m = 0;
+    for (int j = t; j < n; j++) {
+      if (key[z][j] != mine) continue;
+      if (touch[z][j]) r.y |= kRecFirst;
+      (m < 4 ? r.z : r.w) |= (int)((unsigned)j << (8 * (m & 3)));
+      m++;
+    }
+    r.y |= m << kRecCountShift;
+    recs[ptr[z * (gridDim.x + 1) + li] + at] = r;
+  }
+}
+
+// The records of all chunks; the schedule's own arrays are on the device already.
+static cudaError_t chunk_records(gf_assembler* a, const std::vector<uint8_t>& bcmask) {
+  const Schedule& s = a->sched;
+  const int nc = s.nchunks;
+  // one table: elemIndMap, first touches, constrained DOFs, records per chunk
+  const size_t ne = s.first_touch.size(), words = 17 * ne + (bcmask.size() + 3) / 4;
+  DevBuf<int32_t> d_table;
+  cudaError_t e = cudaSuccess;
+  auto up = [&](cudaError_t x) {
+    if (e == cudaSuccess) e = x;
   };
-  std::vector<std::thread> th;
-  for (int t = 1; t < nt; t++) th.emplace_back(work, t);
-  work(0);
-  for (auto& x : th) x.join();
-  for (int li = 0; li < s.nchunks; li++) {
-    bptr[li + 1] += bptr[li];
-    nptr[li + 1] += nptr[li];
-  }
-  brec.reserve(bptr.back());
-  nrec.reserve(nptr.back());
-  for (auto& part : parts) {
-    brec.insert(brec.end(), part.brec.begin(), part.brec.end());
-    nrec.insert(nrec.end(), part.nrec.begin(), part.nrec.end());
-  }
+  auto launch = [&](const int32_t* ptr, int4* recs) {
+    if (e != cudaSuccess) return;
+    const int32_t* t = d_table.p;
+    chunk_records_kernel<<<nc, 16 * kChunkSize>>>(
+        a->d_chunk_start.p, a->d_sorder.p, a->d_sconn.p, t,
+        reinterpret_cast<const uint32_t*>(t + 16 * ne),
+        reinterpret_cast<const uint8_t*>(t + 17 * ne), ptr, d_table.p + words, recs);
+    ::gf::count_launch();
+    up(cudaGetLastError());
+  };
+  up(d_table.alloc(words + nc));
+  auto put = [&](size_t at, const void* src, size_t bytes) {
+    if (e == cudaSuccess) up(cudaMemcpy(d_table.p + at, src, bytes, cudaMemcpyHostToDevice));
+  };
+  put(0, a->emap.data(), sizeof(int32_t) * 16 * ne);
+  put(16 * ne, s.first_touch.data(), sizeof(uint32_t) * ne);
+  put(17 * ne, bcmask.data(), bcmask.size());
+  launch(nullptr, nullptr);
+  std::vector<int32_t> n(nc), ptr(2 * (size_t)(nc + 1), 0);
+  if (e == cudaSuccess)
+    up(cudaMemcpy(n.data(), d_table.p + words, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost));
+  for (int z = 0, at = 0; z < 2; z++)
+    for (int li = 0; li <= nc; li++) {
+      ptr[(size_t)z * (nc + 1) + li] = at;
+      if (li < nc) at += z ? n[li] >> 16 : n[li] & 0xffff;
+    }
+  up(a->d_rptr.upload(ptr));
+  up(a->d_recs.alloc(ptr.back()));
+  launch(a->d_rptr.p, a->d_recs.p);
+  if (e == cudaSuccess) up(cudaStreamSynchronize(nullptr));  // the table ends here
+  return e;
 }
 
 struct AsmParams {
@@ -730,10 +767,9 @@ static AsmParams asm_params(gf_assembler* a, double* values, double* res, int fl
   P.chunk_start = a->d_chunk_start.p;
   P.thick_nat = thick_nat;
   P.sorder = a->d_sorder.p;
-  P.brec = a->d_brec.p;
-  P.bptr = a->d_bptr.p;
-  P.nrec = a->d_nrec.p;
-  P.nptr = a->d_nptr.p;
+  P.brec = P.nrec = a->d_recs.p;
+  P.bptr = a->d_rptr.p;
+  P.nptr = a->d_rptr.p + a->sched.nchunks + 1;
   P.values = values;
   P.res = res;
   P.energy_part = a->d_energy_part.p;
@@ -867,6 +903,7 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
   int dev_count = 0;
   if (cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count == 0) return GF_NO_DEVICE;
 
+  const auto t_setup = std::chrono::steady_clock::now();
   gf_assembler* a = new gf_assembler();
   a->nnodes = nn;
   a->nelem = ne;
@@ -925,9 +962,6 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
   }
   std::vector<uint8_t> bcmask(nn, 0);
   for (int i = 0; i < d->num_bcs; i++) bcmask[d->bcs[i] / 6] |= (uint8_t)(1u << (d->bcs[i] % 6));
-  std::vector<int4> brec, nrec;
-  std::vector<int32_t> bptr, nptr;
-  chunk_records(*d, a->emap, s, bcmask, brec, bptr, nrec, nptr);
   // BC entry list (solver order): rows of constrained DOFs and the matching columns
   std::vector<int32_t> ent;
   const Pattern& P = a->pat;
@@ -963,10 +997,6 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
   up(a->d_bcs.upload(a->bcs));
   up(a->d_sconn.upload(sconn));
   up(a->d_smat.upload(smat));
-  up(a->d_brec.upload(brec));
-  up(a->d_bptr.upload(bptr));
-  up(a->d_nrec.upload(nrec));
-  up(a->d_nptr.upload(nptr));
   up(a->d_sthick.upload(sthick));
   up(a->d_sorder.upload(s.order));
   up(a->d_chunk_start.upload(s.chunk_start));
@@ -976,10 +1006,16 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
   up(a->d_bc_entries.upload(ent));
   up(a->d_energy_part.alloc(s.nchunks + 1));
   up(a->d_diag.upload(diag));
+  if (st == GF_OK) {
+    const auto t_rec = std::chrono::steady_clock::now();
+    up(chunk_records(a, bcmask));
+    a->records_ms = ms_since(t_rec);
+  }
   if (st != GF_OK) {
     delete a;
     return st;
   }
+  a->setup_ms = ms_since(t_setup);
   *out = a;
   return GF_OK;
 }
@@ -1036,6 +1072,13 @@ gf_status gf_assembler_setup_info(const gf_assembler* a, int32_t* pattern_on_gpu
   if (!a) return GF_INVALID_ARG;
   if (pattern_on_gpu) *pattern_on_gpu = (a->sym_flags & 1) ? 1 : 0;
   if (elem_map_on_gpu) *elem_map_on_gpu = (a->sym_flags & 2) ? 1 : 0;
+  return GF_OK;
+}
+
+gf_status gf_assembler_setup_times(const gf_assembler* a, double* records_ms, double* setup_ms) {
+  if (!a) return GF_INVALID_ARG;
+  if (records_ms) *records_ms = a->records_ms;
+  if (setup_ms) *setup_ms = a->setup_ms;
   return GF_OK;
 }
 

@@ -218,6 +218,7 @@ int build_schedule(int nelem, int nnodes, const int32_t* conn, const std::vector
 struct gf_assembler {
   int nnodes = 0, nelem = 0, nbcs = 0;
   int sym_flags = 0;                // bit 0: node pattern, bit 1: elemIndMap computed on the GPU
+  double records_ms = 0.0, setup_ms = 0.0;  // host wall time of the chunk records / of the setup
   gf::Pattern pat0;                 // natural pattern
   gf::Pattern pat;                  // solver-order pattern
   std::vector<int32_t> perm, iperm;
@@ -232,8 +233,8 @@ struct gf_assembler {
   // device: schedule-ordered element data, and the blocks and nodes that each
   // chunk of elements contributes to
   gf::DevBuf<int32_t> d_sconn, d_smat;
-  gf::DevBuf<int4> d_brec, d_nrec;
-  gf::DevBuf<int32_t> d_bptr, d_nptr;
+  gf::DevBuf<int4> d_recs;          // block records of all chunks, then their node records
+  gf::DevBuf<int32_t> d_rptr;       // where each chunk's block records begin, then its node records
   gf::DevBuf<double> d_sthick;
   gf::DevBuf<int32_t> d_sorder;     // schedule position -> element
   gf::DevBuf<int32_t> d_chunk_list, d_chunk_start;

@@ -134,6 +134,10 @@ gf_status gf_assembler_create(const gf_mesh_desc* desc, gf_assembler** out);
  * NULL. The node ordering and the scatter colouring are host algorithms. */
 gf_status gf_assembler_setup_info(const gf_assembler* a, int32_t* pattern_on_gpu,
                                   int32_t* elem_map_on_gpu);
+/* Wall time (ms) of gf_assembler_create, and of the part of it that builds the
+ * records of the blocks and nodes that each chunk of elements contributes to.
+ * Any pointer may be NULL. No reference counterpart. */
+gf_status gf_assembler_setup_times(const gf_assembler* a, double* records_ms, double* setup_ms);
 gf_status gf_order_nodes(const gf_mesh_desc* desc, int32_t* perm);
 gf_status gf_assembler_destroy(gf_assembler* a);
 /* get_num_nodes / get_num_elements / get_num_vars (include/assembler.h:117-118, :309-310) */
