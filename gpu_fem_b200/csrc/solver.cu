@@ -2105,13 +2105,26 @@ struct gf_precond {
 };
 
 namespace gf {
-// Chunk stream of one triangle (layout described at TriDesc).
-static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bool upper) {
+// The chunks of one triangle (layout described at TriDesc): their rows, split
+// over the CTAs.
+struct TriPlan {
+  int nsplit, capb, capr, nch;
+  long long real = 0;                        // stored blocks
+  std::vector<int32_t> chunk_of, grow;       // of a row: its chunk and its number in it
+  std::vector<std::vector<int32_t>> hrows;   // rows of half chunk h * nch + c
+  // bytes of a half chunk ahead of its values: two int4 headers, row records
+  // {row, first block, blocks, row index in the chunk}, the near list, the far
+  // list and rows of the next half chunk, then (16-byte aligned) values
+  static int64_t head_bytes(int64_t rows, int64_t near, int64_t far1, int64_t rows1) {
+    return (32 + 16 * rows + 8 * near + 8 * far1 + 4 * rows1 + 15) & ~(int64_t)15;
+  }
+};
+static cudaError_t plan_tri(const gf_precond* p, const std::vector<int32_t>& diag, bool upper,
+                            TriPlan& t) {
   const Pattern& P = p->pat;
   const int n = P.n;
   const std::vector<int32_t>& lv = upper ? p->lvU : p->lvL;
   const int nlev = upper ? p->nlevU : p->nlevL;
-  const size_t vs = p->prec == GF_PREC_FP32 ? 4 : 8;
   auto cnt = [&](int i) { return upper ? P.rowp[i + 1] - diag[i] : diag[i] - P.rowp[i]; };
   std::vector<int32_t> ptr(nlev + 1, 0), rows(n);
   for (int i = 0; i < n; i++) ptr[lv[i] + 1]++;
@@ -2186,7 +2199,7 @@ static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bo
   const int nch = (int)ck.size() - 1;
   // split every chunk's rows over the CTAs: each row goes to the half with
   // fewer blocks so far (ties: fewer rows), within capr rows a half
-  std::vector<int32_t> half(n), chunk_of(n), grow(n);
+  std::vector<int32_t> chunk_of(n), grow(n);
   std::vector<std::vector<int32_t>> hrows((size_t)kSweepCta * nch);  // [h * nch + c]
   for (int c = 0; c < nch; c++) {
     int hb[kSweepCta] = {0}, hr[kSweepCta] = {0};
@@ -2196,7 +2209,6 @@ static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bo
       for (int q = 1; q < nsplit; q++)
         if (hr[h] == capr || (hr[q] < capr && (hb[q] < hb[h] || (hb[q] == hb[h] && hr[q] < hr[h]))))
           h = q;
-      half[i] = h;
       chunk_of[i] = c;
       grow[i] = k - ck[c];
       hb[h] += cnt(i);
@@ -2206,6 +2218,52 @@ static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bo
     for (int h = 0; h < kSweepCta; h++)
       if (hb[h] > capb || hr[h] > capr) return cudaErrorInvalidValue;
   }
+  t.nsplit = nsplit;
+  t.capb = capb;
+  t.capr = capr;
+  t.nch = nch;
+  t.real = real;
+  t.chunk_of.swap(chunk_of);
+  t.grow.swap(grow);
+  t.hrows.swap(hrows);
+  return cudaSuccess;
+}
+// Bytes of a plan's largest half chunk, from counts alone.
+static int tri_stage(const gf_precond* p, const std::vector<int32_t>& diag, bool upper,
+                     const TriPlan& t) {
+  const Pattern& P = p->pat;
+  const int nch = t.nch;
+  const int64_t vs = p->prec == GF_PREC_FP32 ? 4 : 8;
+  int64_t stage = 0;
+  for (int h = 0; h < kSweepCta; h++) {
+    // of the half chunk behind this one: rows, blocks solved before the chunk ahead
+    int64_t rows1 = 0, far1 = 0;
+    for (int c = nch - 1; c >= 0; c--) {
+      const auto& rows = t.hrows[(size_t)h * nch + c];
+      int64_t near = 0, far = 0;
+      for (int i : rows)
+        for (int jp = upper ? diag[i] + 1 : P.rowp[i]; jp < (upper ? P.rowp[i + 1] : diag[i]); jp++)
+          (t.chunk_of[P.cols[jp]] == c - 1 ? near : far)++;
+      const int64_t b = near + far + (upper ? (int64_t)rows.size() : 0);
+      stage = std::max(stage, TriPlan::head_bytes((int64_t)rows.size(), near, far1, rows1) +
+                                  36 * vs * std::max<int64_t>(4, (b + 3) & ~(int64_t)3));
+      rows1 = (int64_t)rows.size();
+      far1 = far;
+    }
+  }
+  return (int)stage;
+}
+// Chunk stream of one triangle.
+static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bool upper) {
+  const Pattern& P = p->pat;
+  const int n = P.n;
+  const size_t vs = p->prec == GF_PREC_FP32 ? 4 : 8;
+  TriPlan plan;
+  if (const cudaError_t bad = plan_tri(p, diag, upper, plan)) return bad;
+  const int nch = plan.nch;
+  const auto &chunk_of = plan.chunk_of, &grow = plan.grow;
+  const auto& hrows = plan.hrows;
+  auto cnt = [&](int i) { return upper ? P.rowp[i + 1] - diag[i] : diag[i] - P.rowp[i]; };
   // per half chunk: stored blocks (padded), and where each block's x comes
   // from. Near: row solved by the previous chunk (either CTA; ring position
   // = its row index within that chunk); far: solved earlier (global row).
@@ -2239,16 +2297,13 @@ static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bo
   for (int h = 0; h < kSweepCta; h++)
     if (!farl[(size_t)h * nch].empty() || !nearl[(size_t)h * nch].empty())
       return cudaErrorInvalidValue;  // level 0 depends on nothing
-  // byte layout of half chunk (h, c): two int4 headers, row records {row,
-  // first block, blocks, row index in the chunk}, the near list, the far
-  // list and rows of half chunk (h, c+1), then (16-byte aligned) values.
-  // Half h's chunks are contiguous; off[h * (nch + 1) + c] is their start.
+  // half h's chunks are contiguous; off[h * (nch + 1) + c] is the start of half chunk (h, c)
   auto pre = [&](int h, int c) {
     const size_t hc = (size_t)h * nch + c;
-    const int64_t nr = (int64_t)hrows[hc].size();
-    const int64_t nf1 = c + 1 < nch ? (int64_t)farl[hc + 1].size() / 2 : 0;
-    const int64_t nr1 = c + 1 < nch ? (int64_t)hrows[hc + 1].size() : 0;
-    return (32 + 16 * nr + 4 * (int64_t)nearl[hc].size() + 8 * nf1 + 4 * nr1 + 15) & ~(int64_t)15;
+    const bool more = c + 1 < nch;
+    return TriPlan::head_bytes((int64_t)hrows[hc].size(), (int64_t)nearl[hc].size() / 2,
+                               more ? (int64_t)farl[hc + 1].size() / 2 : 0,
+                               more ? (int64_t)hrows[hc + 1].size() : 0);
   };
   std::vector<int64_t> off((size_t)kSweepCta * (nch + 1), 0);
   size_t nslots = 0;
@@ -2313,12 +2368,12 @@ static cudaError_t build_tri(gf_precond* p, const std::vector<int32_t>& diag, bo
   // right-hand side and its result (each x entry is read once, however many
   // blocks multiply it)
   gf_precond::Tri& t = p->tri[upper ? 1 : 0];
-  t.nsplit = nsplit;
-  t.abytes = real * (36 * (long long)vs + 4) + (long long)n * (4 + 48 + 48) + 4;
+  t.nsplit = plan.nsplit;
+  t.abytes = plan.real * (36 * (long long)vs + 4) + (long long)n * (4 + 48 + 48) + 4;
   t.nch = nch;
   t.stage = stage;
-  t.capb = capb;
-  t.capr = capr;
+  t.capb = plan.capb;
+  t.capr = plan.capr;
   t.nslots = nslots;
   cudaError_t e = cudaSuccess;
   auto up = [&](cudaError_t x) {
@@ -3700,28 +3755,28 @@ gf_status gf_precond_create_ex(gf_assembler* a, int32_t fill_level, int32_t prec
       const int k = p->pat.cols[kp];
       p->fwork += p->pat.rowp[k + 1] - diag[k];
     }
+  bool refused = false;
   for (int w = 0; w < 2 && e == cudaSuccess; w++) {
     bool df = false;
     if (sweep == GF_SWEEP_DATAFLOW) e = build_df(p, diag, w == 1, &df);
     // the factors that are refused for their longest row are those that the
     // chunked level sweep cannot stage, whichever sweep solves them: short
-    // rows always fit, others are laid out to see
+    // rows always fit, for others its chunks are counted (150x140 plate,
+    // complete factor, FP64: laid out instead, they took 1,000 of 1,090 ms of
+    // setup beside the pattern)
     if (sweep == GF_SWEEP_AUTO) {
       int most = 0;
       for (int i = 0; i < n; i++)
         most = std::max(most, w ? p->pat.rowp[i + 1] - diag[i] : diag[i] - p->pat.rowp[i]);
       if (most > kRingRowAlways) {
-        e = build_tri(p, diag, w == 1);
-        if (e == cudaSuccess && sweep_smem(p, w) > kSweepSmemMax) break;
+        TriPlan plan;
+        e = plan_tri(p, diag, w == 1, plan);
+        if (e != cudaSuccess) break;
+        refused = sweep_smem_bytes(tri_stage(p, diag, w == 1, plan), plan.capb, plan.capr) >
+                  kSweepSmemMax;
+        if (refused) break;
       }
-      if (e == cudaSuccess) e = build_ring(p, diag, w == 1, &df);
-      if (df) {  // the chunked stream, where it was built
-        gf_precond::Tri& t = p->tri[w];
-        t.off.release();
-        t.vpos.release();
-      } else if (e == cudaSuccess && most > kRingRowAlways) {
-        continue;
-      }
+      e = build_ring(p, diag, w == 1, &df);
     }
     if (e == cudaSuccess && !df) {
       if (sweep == GF_SWEEP_DATAFLOW) {
@@ -3736,7 +3791,7 @@ gf_status gf_precond_create_ex(gf_assembler* a, int32_t fill_level, int32_t prec
   auto fits = [&](int w) {
     return sweep_smem(p, w) <= kSweepSmemMax;
   };
-  if (e == cudaSuccess && !(fits(0) && fits(1))) {
+  if (refused || (e == cudaSuccess && !(fits(0) && fits(1)))) {
     set_last_error_text("gf_precond_create: the ILU(" + std::to_string(fill_level) +
                         ") factor has rows too long for the triangular sweep's "
                         "shared-memory stage; use a lower fill level");
