@@ -111,6 +111,7 @@ SIGNATURES = {
     "gf_precond_info": (_I, [_P, _PI, _PI, _PI]),
     "gf_precond_status": (_I, [_P, _P]),
     "gf_precond_layout": (_I, [_P, _PI, _PI, _PI, _PI, _PI]),
+    "gf_precond_sweep_layout": (_I, [_P, _I, _PI, _PI, _PI]),
     "gf_precond_factor_layout": (_I, [_P, _PI, _PI]),
     "gf_batch_set_scatter": (_I, [_P, C.c_int32]),
     "gf_assembler_setup_info": (_I, [_P, _PI, _PI]),

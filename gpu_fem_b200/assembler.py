@@ -406,6 +406,17 @@ class ILUk_Preconditioner:
         return {"nsplit_L": v[0].value, "nsplit_U": v[1].value, "fac_ctas": v[2].value,
                 "chunks_L": v[3].value, "chunks_U": v[4].value}
 
+    def sweep_layout(self):
+        """Per triangle: kernel ("chunked", "dataflow" or "ring"), CTAs and
+        groups of warps (gf_precond_sweep_layout)."""
+        out = {}
+        for u, tri in enumerate("LU"):
+            v = [C.c_int32() for _ in range(3)]
+            check(L.lib().gf_precond_sweep_layout(self.h, u, *[C.byref(x) for x in v]),
+                  "sweep_layout")
+            out[tri] = (("chunked", "dataflow", "ring")[v[0].value], v[1].value, v[2].value)
+        return out
+
     def factor_layout(self):
         """Rows whose values / whose column -> slot map the factorization keeps
         in shared memory (gf_precond_factor_layout)."""

@@ -3871,6 +3871,19 @@ gf_status gf_precond_sweeps(const gf_precond* p, int32_t* kind_L, int32_t* kind_
   return GF_OK;
 }
 
+gf_status gf_precond_sweep_layout(const gf_precond* p, int32_t upper, int32_t* kernel,
+                                  int32_t* ctas, int32_t* groups) {
+  if (!p || upper < 0 || upper > 1) return GF_INVALID_ARG;
+  const gf_precond::Tri& t = p->tri[upper];
+  if (kernel)
+    *kernel = t.kind == TRI_RING       ? GF_SWEEP_KERNEL_RING
+              : t.kind == TRI_DATAFLOW ? GF_SWEEP_KERNEL_DATAFLOW
+                                       : GF_SWEEP_KERNEL_CHUNKED;
+  if (ctas) *ctas = t.nsplit;
+  if (groups) *groups = t.kind == TRI_RING ? t.groups : 1;
+  return GF_OK;
+}
+
 gf_status gf_precond_status(gf_precond* p, void* stream) {
   if (!p) return GF_INVALID_ARG;
   if (!p->self) return GF_OK;  // nothing has run

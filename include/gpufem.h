@@ -323,6 +323,19 @@ gf_status gf_precond_setup_info(const gf_precond* p, int32_t* symbolic_on_gpu, d
                                 double* setup_ms);
 gf_status gf_precond_layout(const gf_precond* p, int32_t* nsplit_L, int32_t* nsplit_U,
                             int32_t* fac_ctas, int32_t* chunks_L, int32_t* chunks_U);
+/* The kernel that solves a triangle (upper: 0 L, 1 U), the CTAs that share its
+ * levels' rows (1, 2 or 4) and the groups of warps that take its levels in
+ * turn (2 to 4 in the ring sweep, else 1). gf_precond_layout and
+ * gf_precond_sweeps report what a caller chose: the ring sweep is one of the
+ * level-ordered kernels there, and any cluster counts as 2. Any pointer may be
+ * NULL. No reference counterpart. */
+enum {
+  GF_SWEEP_KERNEL_CHUNKED = 0,
+  GF_SWEEP_KERNEL_DATAFLOW = 1,
+  GF_SWEEP_KERNEL_RING = 2
+};
+gf_status gf_precond_sweep_layout(const gf_precond* p, int32_t upper, int32_t* kernel,
+                                  int32_t* ctas, int32_t* groups);
 /* Rows of the factor whose values (at most 80 blocks) and whose column -> slot
  * map (at most 1024 columns from the first to the last) the factorization
  * keeps in shared memory; the others are updated, or searched, in global

@@ -21,16 +21,18 @@ from gpu_fem_b200 import mesh as M
 
 pytestmark = pytest.mark.gpu
 
-# two CTAs, four CTAs, levels of one row at both ends of the plate, and a
-# triangle of 80,601 rows (its later levels are more than a barrier can count)
-CASES = {"two": (200, 60, 8, 0), "four": (256, 128, 6, 0), "tail": (200, 60, 8, 20),
-         "long": (400, 200, 2, 0)}
+# separate plates, nx, ny, fill level, rows of a strip one element wide: two
+# CTAs, four CTAs, levels of one row at both ends of the sweep, and a triangle of
+# 80,601 rows (its later levels are more than a barrier can count)
+FULL = 0x7FFFFFFF
+CASES = {"two": (2, 100, 6, FULL, 0), "four": (1, 256, 128, 6, 0), "tail": (1, 200, 60, 8, 20),
+         "long": (1, 400, 200, 2, 0)}
 
 
 def _factored(case, precision):
     import torch
     from gpu_fem_b200.assembler import ElementAssembler, ILUk_Preconditioner, createBsrMat
-    nx, ny, fill, tail = CASES[case]
+    parts, nx, ny, fill, tail = CASES[case]
     m = M.plate(nx, ny + tail, 1.0, 0.5, lambda x, y: 0.006 + 0 * x, "x0",
                 lambda q: 1e3 + 0 * q[:, 0])
     if tail:  # beyond row ny only the last column of elements
@@ -43,6 +45,12 @@ def _factored(case, precision):
         bcs = m.bcs[new[m.bcs // 6] >= 0]
         m.bcs = (6 * new[bcs // 6] + bcs % 6).astype(np.int32)
         m.conn, m.xpts = new[m.conn].astype(np.int32), m.xpts[nodes]
+    n = m.num_nodes
+    m = M.ShellMesh(np.concatenate([m.conn + k * n for k in range(parts)]).astype(np.int32),
+                    np.concatenate([m.xpts + [0.0, 2.0 * k, 0.0] for k in range(parts)]),
+                    np.tile(m.thick, parts),
+                    np.concatenate([m.bcs + 6 * n * k for k in range(parts)]).astype(np.int32),
+                    np.zeros(6 * n * parts))
     A = ElementAssembler.from_mesh(m, ordering="natural")
     K = createBsrMat(A)
     A.add_jacobian(None, K, fuse_bcs=True)
@@ -59,8 +67,9 @@ def test_ctas_that_give_up_leave_quietly(case, precision):
     from gpu_fem_b200 import _lib as L
     lib = L.lib()
     m, P = _factored(case, precision)
-    lay = P.layout()
-    assert (lay["nsplit_L"], lay["nsplit_U"]) == (2, 2)  # both split
+    lay = P.sweep_layout()
+    ctas = lay["L"][1] + lay["U"][1]
+    assert ctas == (4 if case == "two" else 8), lay
 
     def exits():
         g, q = C.c_int32(), C.c_int32()
@@ -76,8 +85,8 @@ def test_ctas_that_give_up_leave_quietly(case, precision):
         P.apply(r, z1)
         assert P.status() == L.GF_TIMEOUT
         gave_up, quiet = exits()
-        # every CTA of both sweeps' clusters of two or four
-        assert gave_up in (4, 6, 8) and quiet == gave_up
+        # every CTA of both sweeps' clusters
+        assert gave_up == ctas and quiet == gave_up
         L.check(lib.gf_test_set_waits(1, 0), "set_waits")
         for _ in range(20):
             P.apply(r, z1)
