@@ -313,8 +313,7 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
 // 2,300, stores 640, release 970, the rest is the flag's way to the waiting
 // warp. Alone, before -> now (B200): 256x128, ILU(6) 11.7 -> 6.4 ms; 61x37,
 // ILU(8) 3.9 -> 2.0 ms; the 64-plate batch 38 -> 32 ms.
-constexpr int kFacWarps = 8;      // warps a CTA counts for when CTAs are shared out
-constexpr int kFacWarpsMax = 8;  // warps of a CTA at most (its shared memory decides)
+constexpr int kFacWarps = 8;      // warps of a CTA
 constexpr int kFacVals = 80;      // row blocks whose values are staged at most
 constexpr int kFacSteps = 64;     // steps of a row that are staged
 constexpr int kFacMap = 1024;     // column span of a row whose column -> slot map is kept
@@ -322,10 +321,11 @@ constexpr uint16_t kFacNone = 0xffff;  // map entry of a column that the row doe
 constexpr size_t kFacSmemMax = 226 * 1024;
 // per warp: values of `vals` blocks and one more that padding reads, the
 // steps, two lists of updates and the column map
-__host__ __device__ inline size_t fac_warp_smem(int vals) {
+__host__ __device__ constexpr size_t fac_warp_smem(int vals) {
   return sizeof(double) * 36 * ((size_t)vals + 1) + sizeof(int4) * kFacSteps + sizeof(int2) * 64 +
          sizeof(uint16_t) * kFacMap;
 }
+static_assert(kFacWarps * fac_warp_smem(kFacVals) <= kFacSmemMax, "the warps' rows fit a CTA");
 // Whether the column -> slot map of a row from column c0 to column c1 is kept
 // (otherwise every block of U(k) is searched for in the row's columns in global
 // memory: 130x128 plate, complete factor, rows of 263 blocks, 390 ms searched,
@@ -553,10 +553,9 @@ __device__ __forceinline__ bool factor_row(const RowValues<STAGED> R, const int4
 
 // cta_prob[blockIdx.x]: the problem a CTA works on; grab[p]: problem p's row
 // counter (zero at launch). vals: blocks of a row that are staged.
-__global__ void __launch_bounds__(kFacWarpsMax * 32) bfactor_df(const ProbDev* __restrict__ P,
-                                                               const int32_t* __restrict__ cta_prob,
-                                                               int* __restrict__ grab, int epoch,
-                                                               int vals, SweepCtl* ctl) {
+__global__ void __launch_bounds__(kFacWarps * 32)
+    bfactor_df(const ProbDev* __restrict__ P, const int32_t* __restrict__ cta_prob,
+               int* __restrict__ grab, int epoch, int vals, SweepCtl* ctl) {
   extern __shared__ __align__(16) unsigned char fsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* ws = fsm + (unsigned)warp * (unsigned)fac_warp_smem(vals);
@@ -2811,8 +2810,8 @@ struct gf_batch {
   DevBuf<double> d_tmp, d_b, d_x;
   int nchunks = 0;
   DevBuf<int32_t> d_cprob, d_pstart;
-  int fac_grid = 0;                  // CTAs of the dataflow factorization,
-  int fac_vals = 0, fac_warps = 0;   // row blocks staged per warp, warps of a CTA
+  int fac_grid = 0;                  // CTAs of the dataflow factorization
+  int fac_vals = 0;                  // row blocks staged per warp
   DevBuf<int32_t> d_fcta, d_fgrab;   // problem of each CTA; per-problem row counters
   DevBuf<int64_t> d_clo, d_chi;
   DevBuf<PermEntry> d_perm_b, d_perm_x, d_perm_out;
@@ -3077,11 +3076,10 @@ static gf_status batch_build(gf_batch* B) {
     std::vector<int32_t> cta_prob;
     fac_plan(B->pcs, ctas, cta_prob);
     B->fac_grid = (int)cta_prob.size();
-    // stage the longest row (up to kFacVals blocks); as many warps as then fit
+    // stage the longest row (up to kFacVals blocks)
     int most = 8;
     for (auto* p : B->pcs) most = std::max(most, p->maxrow);
     B->fac_vals = std::min(most, kFacVals);
-    B->fac_warps = (int)std::min<size_t>(kFacWarpsMax, kFacSmemMax / fac_warp_smem(B->fac_vals)) & ~1;
     up(B->d_fcta.upload(cta_prob));
     up(B->d_fgrab.alloc(np));
   }
@@ -3327,9 +3325,8 @@ static gf_status batch_factor(gf_batch* B, cudaStream_t st) {
     ::gf::count_launch();
     GF_CUDA(cudaFuncSetAttribute(bfactor_df, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kFacSmemMax));
-    bfactor_df<<<(unsigned)B->fac_grid, B->fac_warps * 32,
-                 B->fac_warps * fac_warp_smem(B->fac_vals), st>>>(
-        B->d_desc.p, B->d_fcta.p, B->d_fgrab.p, epoch, B->fac_vals, B->d_ctl.p);
+    bfactor_df<<<(unsigned)B->fac_grid, kFacWarps * 32, kFacWarps * fac_warp_smem(B->fac_vals),
+                 st>>>(B->d_desc.p, B->d_fcta.p, B->d_fgrab.p, epoch, B->fac_vals, B->d_ctl.p);
   }
   GF_CHECK_LAUNCH();
   for (int k = 0; k < B->np; k++) {
