@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kAsmThreads, 4)
 struct ResSlot {
   double X[12], U[24], fn[12];
   double d[4][3];       // director displacements theta x fn of the nodes
-  double drill[4];      // nodal drill strains, then their adjoints per point
+  double drill[4];      // nodal drill strains
   double V[4][15];      // per point: adjoints of u_xi, u_eta, d_xi, d_eta, d
   double G[4][5];       // ... of the tying strains g11 g22 g12 g23 g13
   double S8[4];         // ... of the drill strain
@@ -638,7 +638,6 @@ __device__ __forceinline__ void residual_chunk(const AsmParams& P, int li, ResSl
         rd[c] += Nx * V[6 + c] + Ne * V[9 + c] + N * V[12 + c];
       }
     }
-    e.drill[q] = dn;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double X = 0.5 * (e.X[6 * ja + 3 + c] - e.X[6 * ja + c]);
