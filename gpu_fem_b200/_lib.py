@@ -118,6 +118,7 @@ SIGNATURES = {
     "gf_assembler_setup_times": (_I, [_P, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "gf_precond_setup_info": (_I, [_P, _PI, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "gf_test_set_waits": (_I, [C.c_ulonglong, _I]),
+    "gf_test_kept_blocks": (_I, []),
     "gf_test_sweep_exits": (_I, [_P, _PI, _PI]),
     "gf_precond_get": (_I, [_P, _PI, _PI, _PD]),
     "gf_solve_opts_default": (None, [C.POINTER(gf_solve_opts)]),

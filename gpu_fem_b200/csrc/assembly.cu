@@ -1015,11 +1015,13 @@ gf_status gf_assembler_create(const gf_mesh_desc* d, gf_assembler** out) {
     return st;
   }
   a->setup_ms = ms_since(t_setup);
+  count_assemblers(1);
   *out = a;
   return GF_OK;
 }
 
 gf_status gf_assembler_destroy(gf_assembler* a) {
+  if (a) count_assemblers(-1);
   delete a;
   return GF_OK;
 }

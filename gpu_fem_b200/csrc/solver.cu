@@ -2717,7 +2717,10 @@ static size_t sweep_smem(const gf_precond* p, int which) {
 // milliseconds to get and to free, so a batch hands its block on: blocks for
 // up to kPollProblems problems go to a list that keeps at most kPollKept of
 // them (4 KB each) and frees the others. A block belongs to one batch at a
-// time, and a batch's solves have ended when it is destroyed.
+// time, and a batch's solves have ended when it is destroyed. The list lives
+// as long as any assembler does: with the last one it is given back, so that
+// a program that has destroyed its objects holds nothing (and may reset its
+// device).
 constexpr int kPollProblems = 64, kPollKept = 8;
 struct PollBlock {
   void* mem = nullptr;
@@ -2726,6 +2729,7 @@ struct PollBlock {
 };
 static std::mutex g_poll_mu;
 static std::vector<PollBlock> g_poll_kept;
+static int g_poll_users = 0;  // assemblers alive
 
 struct SolvePoll {
   PollBlock blk;
@@ -2780,7 +2784,7 @@ struct SolvePoll {
       if (x) cudaEventSynchronize(x);  // no step of an aborted solve writes here any more
     if (blk.mem && blk.cap == kPollProblems) {
       std::lock_guard<std::mutex> lk(g_poll_mu);
-      if (g_poll_kept.size() < (size_t)kPollKept) {
+      if (g_poll_users > 0 && g_poll_kept.size() < (size_t)kPollKept) {
         g_poll_kept.push_back(blk);
         return;
       }
@@ -2788,6 +2792,18 @@ struct SolvePoll {
     free_block(blk);
   }
 };
+
+namespace gf {
+void count_assemblers(int more) {
+  std::vector<PollBlock> gone;
+  {
+    std::lock_guard<std::mutex> lk(g_poll_mu);
+    g_poll_users += more;
+    if (g_poll_users == 0) gone.swap(g_poll_kept);
+  }
+  for (auto& b : gone) SolvePoll::free_block(b);
+}
+}  // namespace gf
 
 struct gf_batch {
   int np = 0, nrows = 0, maxlevL = 0, maxlevU = 0;
@@ -3896,6 +3912,11 @@ gf_status gf_test_set_waits(unsigned long long wait_ns, int32_t skip_meetings) {
   GF_CUDA(cudaMemcpyToSymbol(g_wait_ns, &w, sizeof(w)));
   GF_CUDA(cudaMemcpyToSymbol(g_skip_meet, &k, sizeof(k)));
   return GF_OK;
+}
+
+int32_t gf_test_kept_blocks(void) {
+  std::lock_guard<std::mutex> lk(g_poll_mu);
+  return (int32_t)g_poll_kept.size();
 }
 
 gf_status gf_test_sweep_exits(const gf_precond* p, int32_t* gave_up, int32_t* quiet) {

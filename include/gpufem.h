@@ -454,6 +454,9 @@ gf_status gf_batch_solve(gf_batch* b, const double* const* d_b, double* const* d
  * it only while no other work of this library runs there, and restore it
  * with gf_test_set_waits(0, 0). No reference counterpart. */
 gf_status gf_test_set_waits(unsigned long long wait_ns, int32_t skip_meetings);
+/* Blocks of pinned host memory (4 KB each, at most 8) that finished solves have
+ * left for later ones; none once the last assembler is destroyed. */
+int32_t gf_test_kept_blocks(void);
 /* Of the sweeps between the last two reads of the preconditioner's device
  * status (gf_precond_status): CTAs of split default sweeps that gave up
  * waiting, and those of them that left with no store in flight to them (all
