@@ -1649,9 +1649,10 @@ __global__ void __launch_bounds__(kDfThreads) bsweep_df(const ProbDev* __restric
       }
       if (__any_sync(0xffffffffu, !okw)) break;
       const int next = q0 + 5;
-      // report progress every kDfWriteBatch positions; the release makes the
-      // slot reads above complete before any warp may overwrite the slots
-      if (next % kDfWriteBatch == 0 || next >= n) {
+      // report progress every kDfWriteBatch positions (the ring has room for
+      // no longer lag than that: build_df); the release makes the slot reads
+      // above complete before any warp may overwrite the slots
+      if (next / kDfWriteBatch != q0 / kDfWriteBatch || next >= n) {
         __syncwarp();
         if (lane == 0) st_release_s32(&wpos[kDfWarps], next >= n ? 0x7fffffff : next);
       }
