@@ -58,8 +58,8 @@ def _args():
                     help="length of the Poisson request stream of the serving run (0 skips it)")
     ap.add_argument("--assembly-case", action="store_true",
                     help="small profiling case: Jacobian assembly (fused BCs) of the 400x200 "
-                         "jittered cantilever plate, 5 times (no JSON line)")
-    ap.add_argument("--sweep-case", choices=["dataflow", "level"], default=None,
+                         "jittered cantilever plate, 5 times, and its residual (no JSON line)")
+    ap.add_argument("--sweep-case", choices=["auto", "dataflow", "level"], default=None,
                     help="small profiling case: the triangular sweeps of one 256x128 plate, "
                          "natural ordering, ILU(6), FP32 factors, applied 5 times with the "
                          "given sweep kernel (no JSON line)")
@@ -103,11 +103,11 @@ def serving_run(seconds):
 
 def assembly_case():
     """Jacobian assembly with fused BCs of the 400x200 plate (80,601 nodes,
-    ~209 MB of block values, above L2), 5 times with the coloured scatter:
-    the small case on which the assembly kernel is profiled. Then prints the
-    event-timed Jacobian with the coloured and the atomic scatter, alone and
-    for the 64-plate batch (one launch per colour over all problems, or one
-    launch with atomics)."""
+    ~209 MB of block values, above L2), 5 times with the coloured scatter, then
+    its residual twice: the small case on which the assembly kernels are
+    profiled. Then prints the event-timed residual and the Jacobian with the
+    coloured and the atomic scatter, alone and for the 64-plate batch (one
+    launch per colour over all problems, or one launch with atomics)."""
     import torch
     from gpu_fem_b200 import mesh as M
     from gpu_fem_b200.assembler import ElementAssembler, ILUk_Preconditioner, createBsrMat
@@ -118,6 +118,8 @@ def assembly_case():
     res = A.createVarsVec()
     for _ in range(5):
         A.add_jacobian(res, K, fuse_bcs=True)
+    for _ in range(2):
+        A.add_residual(res)
     torch.cuda.synchronize()
     print("assembly case", A.get_nnzb())
 
@@ -131,7 +133,8 @@ def assembly_case():
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / reps
 
-    out = {"400x200 coloured ms": timed(lambda: A.add_jacobian(None, K, fuse_bcs=True)),
+    out = {"400x200 residual ms": timed(lambda: A.add_residual(res)),
+           "400x200 coloured ms": timed(lambda: A.add_jacobian(None, K, fuse_bcs=True)),
            "400x200 atomic ms": timed(lambda: A.add_jacobian(None, K, fuse_bcs=True, atomic=True))}
     meshes = M.batch_config4(64)
     asms = [ElementAssembler.from_mesh(mm, ordering="natural") for mm in meshes]
@@ -148,9 +151,9 @@ def sweep_case(kind):
     """One preconditioner (256x128 clamped plate, t = 2 mm, natural ordering,
     ILU(6), FP32 factors, ~150 MB of factor) applied 5 times with the given
     sweep kernel: the small case on which the sweep and factorization kernels
-    are profiled (its levels are large enough that the factorization and the
-    level-synchronous sweeps run on a two-CTA cluster). Prints the mean
-    event-timed apply (both sweeps)."""
+    are profiled (its levels are large enough that the default sweep runs on a
+    cluster of four CTAs, the chunked one on two and the factorization on 128).
+    Prints the mean event-timed apply (both sweeps)."""
     import torch
     from gpu_fem_b200 import mesh as M
     from gpu_fem_b200.assembler import ElementAssembler, ILUk_Preconditioner, createBsrMat
@@ -170,7 +173,7 @@ def sweep_case(kind):
         P.apply(r, z)
     e1.record()
     torch.cuda.synchronize()
-    print("sweep case", kind, P.info(), P.sweeps(), f"{e0.elapsed_time(e1) / 5:.3f} ms per apply",
+    print("sweep case", kind, P.info(), P.sweep_layout(), f"{e0.elapsed_time(e1) / 5:.3f} ms per apply",
           float(z.abs().max()))
 
 

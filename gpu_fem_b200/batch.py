@@ -98,9 +98,10 @@ def factor_work(nrow, inf):
 
 
 # The cost models below only rank candidates against one another. They were
-# fitted to kernels that took about twice as long as the present ones, sweeps
-# (1.2-2.2 -> 0.46-0.9 us a level) and factorization (9 -> 5 us a level) alike,
-# which leaves the ranking as it is.
+# fitted to slower kernels than the present ones: sweeps took 1.2-2.2 us a level
+# (now 0.44-0.83), the factorization 9 (now 5), a GMRES step's other work 150 us.
+# They therefore rate a sweep about a third too dear against a factorization
+# and lean towards higher fills than a fit to the present kernels would.
 def factor_cost_us(nrow, inf, warps=None):
     """One numeric factorization of a problem (microseconds), fitted to B200
     runs of single plates (16^2 to 256^2 elements, fills 1 to 16) on the

@@ -12,11 +12,12 @@
 // problem of a global block row (row_prob), its offset in the batch vector
 // space and its triangular level structure.
 //  * SpMV and the GMRES vector work run over all rows / chunks of the batch.
-//  * Triangular work (the factorization and both sweeps) runs one CTA per
-//    problem: the CTA walks the problem's levels and separates them with
-//    __syncthreads(), so a dependency costs a block barrier (tens of ns)
-//    instead of a device-wide round trip; the problems of a batch run on
-//    different SMs at once.
+//  * A triangular sweep runs one CTA, or the CTAs of one cluster, per problem:
+//    they walk the problem's levels, so a dependency costs a barrier between
+//    warps (or an exchange within the cluster) instead of a device-wide round
+//    trip; the problems of a batch run on different SMs at once.
+//  * The factorization shares the SMs out over the problems; its rows wait for
+//    one another through flags in global memory.
 //
 // GMRES reductions are segmented per problem over fixed 4096-entry chunks
 // aligned to each problem's own vector, with per-problem Arnoldi states, so
@@ -311,8 +312,8 @@ __device__ __forceinline__ bool inv6_cols(double (&m)[6]) {
 // reads the lower part in this launch), released by one lane. Clocks of that
 // chain on a 256x128 plate, ILU(6): operands 1,150, updates 1,300, inverse
 // 2,300, stores 640, release 970, the rest is the flag's way to the waiting
-// warp. Alone, before -> now (B200): 256x128, ILU(6) 11.7 -> 6.4 ms; 61x37,
-// ILU(8) 3.9 -> 2.0 ms; the 64-plate batch 38 -> 32 ms.
+// warp. Alone, before -> now (B200): 256x128, ILU(6) 11.7 -> 6.2 ms; 61x37,
+// ILU(8) 3.6 -> 2.0 ms; 256x256, ILU(12) 22.6 ms; the 64-plate batch 38 -> 30 ms.
 constexpr int kFacWarps = 8;      // warps of a CTA
 constexpr int kFacVals = 80;      // row blocks whose values are staged at most
 constexpr int kFacSteps = 64;     // steps of a row that are staged
@@ -999,7 +1000,9 @@ __global__ void __launch_bounds__(kSweepThreads) bsweep_tma(const ProbDev* __res
 //  - a warp takes a row 16 blocks a pass; lane (j, h) multiplies rows
 //    3h..3h+2 of block j. The values are read once, so they go from L2
 //    straight to registers while the other groups' levels run, and every pass
-//    prefetches as many bytes kRingAhead ahead of its own from HBM into L2;
+//    prefetches from HBM into L2, kRingAhead bytes ahead of itself, a line of
+//    128 bytes for each lane that has values: all that a pass of the same
+//    length takes in FP32, 8/9 of it in FP64, and not U_ii^{-1};
 //  - the 16 partial sums of a row meet in a reduce-scatter of five 64-bit
 //    shuffles (a butterfly over three sums takes twelve);
 //  - rows of more than 16 blocks are shared by several warps.
