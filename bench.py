@@ -266,9 +266,8 @@ def _dist():
 # DRAM bytes (read + write) of a sweep launch over its algorithmic bytes,
 # from an ncu capture of the 256x128 ILU(6) FP32 sweep case (the batch's
 # launches are too large to capture): 81.1 MB / 80.2 MB for L, 86.0 MB /
-# 85.1 MB for U (profiles/bsweep_ring_256x128_ilu6.md). Traffic per
-# launch grows with the blocks streamed, so the bench scales the ratio by its
-# own algorithmic bytes per launch.
+# 85.1 MB for U. Traffic per launch grows with the blocks streamed, so the
+# bench scales the ratio by its own algorithmic bytes per launch.
 SWEEP_TRAFFIC_RATIO = 1.011
 
 # Fill level k and node ordering of each of the 64 problems, as chosen by the

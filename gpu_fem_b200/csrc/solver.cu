@@ -1401,6 +1401,7 @@ __device__ __forceinline__ void ring_sweep(unsigned char* ring, RingShared& sh, 
   if (SPLIT) {
     // From here on nobody sends. A CTA that has not given up has waited for
     // every byte of every level; one that has waits for what it was sent.
+    __syncwarp();  // the barrier is one instruction of a whole warp
     cluster_barrier();
     if (abort_flag) ring_drain(T, rank, gone, xbar, ctl);
   }
