@@ -257,7 +257,7 @@ struct gf_bsr {
 
 namespace gf {
 // one more assembler (or, with -1, one less) is alive: with the last one the
-// host memory that solves hand on is freed
+// host memory that solves hand on is freed but for one block
 void count_assemblers(int more);
 gf_status batch_assemble(BatchAsm*& cache, const std::vector<gf_assembler*>& asms,
                          const std::vector<double*>& values, const double* const* thick, int flags,

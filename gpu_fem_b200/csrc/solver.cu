@@ -2722,15 +2722,34 @@ static size_t sweep_smem(const gf_precond* p, int which) {
 // milliseconds to get and to free, so a batch hands its block on: blocks for
 // up to kPollProblems problems go to a list that keeps at most kPollKept of
 // them (4 KB each) and frees the others. A block belongs to one batch at a
-// time, and a batch's solves have ended when it is destroyed. The list lives
-// as long as any assembler does: with the last one it is given back, so that
-// a program that has destroyed its objects holds nothing (and may reset its
-// device).
+// time, and a batch's solves have ended when it is destroyed. With the last
+// assembler the list is given back but for one block: a program that makes
+// and destroys all its objects for every solve would pay for a new one each
+// time (33x21 plate, FP64: 4.2-5.1 instead of 2.8 ms). A block is handed out
+// only while it is what it was: a device reset frees it behind the list's
+// back, so its memory has to be pinned still and to bear its mark.
 constexpr int kPollProblems = 64, kPollKept = 8;
 struct PollBlock {
   void* mem = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   int device = -1, cap = 0;
+  static size_t bytes(int cap) {
+    return ((sizeof(double) * 2 * cap + sizeof(int) * (3 * (size_t)cap + 2) + 7) & ~(size_t)7) +
+           sizeof(uint64_t);
+  }
+  uint64_t* mark() const {
+    return reinterpret_cast<uint64_t*>(static_cast<char*>(mem) + bytes(cap)) - 1;
+  }
+  uint64_t sign() const {
+    return 0x9e3779b97f4a7c15ull * (uint64_t)reinterpret_cast<uintptr_t>(mem) ^
+           (uint64_t)reinterpret_cast<uintptr_t>(ev[0]);
+  }
+  bool intact() const {
+    cudaPointerAttributes at;
+    const cudaError_t e = cudaPointerGetAttributes(&at, mem);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && at.type == cudaMemoryTypeHost && *mark() == sign();
+  }
 };
 static std::mutex g_poll_mu;
 static std::vector<PollBlock> g_poll_kept;
@@ -2760,24 +2779,26 @@ struct SolvePoll {
     const int cap = std::max(np, kPollProblems);
     if (cap == kPollProblems) {
       std::lock_guard<std::mutex> lk(g_poll_mu);
-      for (size_t k = 0; k < g_poll_kept.size(); k++)
-        if (g_poll_kept[k].device == dev) {
-          blk = g_poll_kept[k];
-          g_poll_kept.erase(g_poll_kept.begin() + k);
-          break;
+      for (size_t k = 0; k < g_poll_kept.size() && !blk.mem;) {
+        if (g_poll_kept[k].device != dev) {
+          k++;
+          continue;
         }
+        if (g_poll_kept[k].intact()) blk = g_poll_kept[k];
+        g_poll_kept.erase(g_poll_kept.begin() + k);
+      }
     }
     if (!blk.mem) {
       blk.device = dev;
       blk.cap = cap;
-      e = cudaHostAlloc(&blk.mem, sizeof(double) * 2 * cap + sizeof(int) * (3 * (size_t)cap + 2),
-                        cudaHostAllocMapped | cudaHostAllocPortable);
+      e = cudaHostAlloc(&blk.mem, PollBlock::bytes(cap), cudaHostAllocMapped | cudaHostAllocPortable);
       for (auto& x : blk.ev)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
       if (e != cudaSuccess) {
         free_block(blk);
         return e;
       }
+      *blk.mark() = blk.sign();
     }
     norms = static_cast<double*>(blk.mem);
     counts = reinterpret_cast<int*>(norms + 2 * np);
@@ -2789,7 +2810,7 @@ struct SolvePoll {
       if (x) cudaEventSynchronize(x);  // no step of an aborted solve writes here any more
     if (blk.mem && blk.cap == kPollProblems) {
       std::lock_guard<std::mutex> lk(g_poll_mu);
-      if (g_poll_users > 0 && g_poll_kept.size() < (size_t)kPollKept) {
+      if (g_poll_kept.size() < (size_t)(g_poll_users > 0 ? kPollKept : 1)) {
         g_poll_kept.push_back(blk);
         return;
       }
@@ -2804,9 +2825,13 @@ void count_assemblers(int more) {
   {
     std::lock_guard<std::mutex> lk(g_poll_mu);
     g_poll_users += more;
-    if (g_poll_users == 0) gone.swap(g_poll_kept);
+    while (g_poll_users == 0 && g_poll_kept.size() > 1) {
+      gone.push_back(g_poll_kept.back());
+      g_poll_kept.pop_back();
+    }
   }
-  for (auto& b : gone) SolvePoll::free_block(b);
+  for (auto& b : gone)
+    if (b.intact()) SolvePoll::free_block(b);
 }
 }  // namespace gf
 

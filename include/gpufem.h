@@ -455,7 +455,7 @@ gf_status gf_batch_solve(gf_batch* b, const double* const* d_b, double* const* d
  * with gf_test_set_waits(0, 0). No reference counterpart. */
 gf_status gf_test_set_waits(unsigned long long wait_ns, int32_t skip_meetings);
 /* Blocks of pinned host memory (4 KB each, at most 8) that finished solves have
- * left for later ones; none once the last assembler is destroyed. */
+ * left for later ones; at most one once the last assembler is destroyed. */
 int32_t gf_test_kept_blocks(void);
 /* Of the sweeps between the last two reads of the preconditioner's device
  * status (gf_precond_status): CTAs of split default sweeps that gave up

@@ -1,9 +1,9 @@
 """Host memory that solves hand on is given back with the last assembler.
 
 A solve follows its problems through a block of pinned memory, which the next
-batch takes over. The blocks are kept only while an assembler is alive, at
-most eight of them; threads that solve at the same time take one each. Counted
-in a process of its own, where no other test's objects are alive.
+batch takes over. While an assembler is alive at most eight blocks are kept,
+afterwards one; threads that solve at the same time take one each. Counted in a
+process of its own, where no other test's objects are alive.
 """
 import os
 import subprocess
@@ -31,6 +31,7 @@ for again in range(2):
     objects = [make() for _ in range(10)]
     torch.cuda.synchronize()
     x = [torch.zeros_like(b) for _ in objects]
+    assert kept() == again, kept()
     direct_solve(*objects[0], b, x[0])
     assert kept() == 1, kept()
     threads = [threading.Thread(target=direct_solve, args=(A, K, b, x[k].zero_()))
@@ -46,7 +47,7 @@ for again in range(2):
     objects.clear()  # K keeps its assembler alive
     assert kept() >= 1, kept()
     del K
-    assert kept() == 0, kept()
+    assert kept() == 1, kept()
 print("ok")
 """
 
